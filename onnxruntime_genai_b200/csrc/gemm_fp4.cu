@@ -38,14 +38,12 @@
 // streaming kernel further down, which keeps the expanded weights in registers.
 #include <cstdlib>
 
-#include <cuda_fp16.h>
-
 #include "gemm_common.cuh"
 #include "kernels.h"
+#include "packed_weights.cuh"
 
 namespace ogb {
 
-constexpr int FP4_RECORD_BYTES = GEMM_BLOCK_N * 32 + GEMM_BLOCK_N * 2;  // 4352
 constexpr int FP4_THREADS = 320;   // warp 0 producer, warp 1 MMA issuer, warps 2..9 expanders (2..5 also run the epilogue)
 constexpr int FP4_DEQ_WARPS = 8;
 
@@ -72,45 +70,6 @@ struct Fp4Cfg {
   static_assert((RAW * FP4_RECORD_BYTES) % 1024 == 0, "swizzled tiles need 1 KiB alignment");
   static_assert(BT * GEMM_BLOCK_N * 4 <= DATA_BYTES, "the parked fp32 tile must fit in the pipeline memory");
 };
-
-__device__ __forceinline__ void fp4_bulk_copy_g2s(void* smem_dst, const void* gsrc, uint32_t bytes, uint64_t* bar) {
-  asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
-               ::"r"(smem_u32(smem_dst)), "l"(gsrc), "r"(bytes), "r"(smem_u32(bar)) : "memory");
-}
-
-// two e2m1 codes (low nibbles of the two halves of `u`) times the block's power-of-two multiplier
-__device__ __forceinline__ uint32_t deq_fp4_pair(uint32_t u, __nv_bfloat162 s2) {
-  uint32_t t = ((u & 0x00070007u) << 6) | ((u & 0x00080008u) << 12);
-  __nv_bfloat162 v = *reinterpret_cast<__nv_bfloat162*>(&t);
-  v = __hmul2(v, s2);
-  return *reinterpret_cast<uint32_t*>(&v);
-}
-
-// fp16 form.  A record word holds eight consecutive k values: byte i = (element i in the low nibble, element 4 + i in the
-// high nibble).  `cvt.rn.f16x2.e2m1x2` turns a byte into the fp16 pair (element i, element 4 + i); two byte permutes put
-// consecutive elements side by side for the K-major tile; one `mul.f16x2` applies the block's power of two.
-// the four bytes of a record word -> four fp16x2 registers: byte i = (k value i, k value 4 + i)
-__device__ __forceinline__ void cvt_e2m1x8_f16(uint32_t word, uint32_t (&h)[4]) {
-  asm("{\n\t.reg .b8 b0, b1, b2, b3;\n\t"
-      "mov.b32 {b0, b1, b2, b3}, %4;\n\t"
-      "cvt.rn.f16x2.e2m1x2 %0, b0;\n\t"
-      "cvt.rn.f16x2.e2m1x2 %1, b1;\n\t"
-      "cvt.rn.f16x2.e2m1x2 %2, b2;\n\t"
-      "cvt.rn.f16x2.e2m1x2 %3, b3;\n\t}"
-      : "=r"(h[0]), "=r"(h[1]), "=r"(h[2]), "=r"(h[3]) : "r"(word));
-}
-__device__ __forceinline__ uint32_t hmul2_bits(uint32_t a, uint32_t b) {
-  __half2 v = __hmul2(*reinterpret_cast<__half2*>(&a), *reinterpret_cast<__half2*>(&b));
-  return *reinterpret_cast<uint32_t*>(&v);
-}
-// eight codes of a record word -> four fp16x2 registers (consecutive k) times the block's multiplier
-__device__ __forceinline__ uint4 deq_fp4_word_f16(uint32_t word, __half2 s2) {
-  const uint32_t s = *reinterpret_cast<uint32_t*>(&s2);
-  uint32_t h[4];
-  cvt_e2m1x8_f16(word, h);       // (k0 k4) (k1 k5) (k2 k6) (k3 k7)
-  return make_uint4(hmul2_bits(__byte_perm(h[0], h[1], 0x5410), s), hmul2_bits(__byte_perm(h[2], h[3], 0x5410), s),
-                    hmul2_bits(__byte_perm(h[0], h[1], 0x7632), s), hmul2_bits(__byte_perm(h[2], h[3], 0x7632), s));
-}
 
 // FP4_WBUF: expanded weight tiles in flight; GROUPS: 1 = all eight expander warps share every k-block (two threads per
 // row), 2 = warps 2..5 take the even k-blocks and warps 6..9 the odd ones (one thread per row).
@@ -145,8 +104,6 @@ gemm_fp4_grouped_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid
   // The tile list is written by the kernel before this one, so nothing is read ahead of it.
   if (p.pdl) pdl_wait();
   if (m_tile >= *p.grp.num_tiles) return;   // uniform over the CTA
-#ifdef OGB_FP4_TRACE
-#endif
   const int row0 = p.grp.tile_row0[m_tile];
   const int rows = p.grp.tile_rows[m_tile];
   const int expert = p.grp.tile_expert[m_tile];
@@ -184,7 +141,7 @@ gemm_fp4_grouped_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid
         const int s = i % RAW;
         mbar_expect_tx(&raw_full[s], FP4_RECORD_BYTES);
         if (w_by_tma) tma_load_2d(raw_ring + s * FP4_RECORD_BYTES, &tmap_w, &raw_full[s], 0, (rec_first + i * n_tiles_per_expert) * (FP4_RECORD_BYTES / 128));
-        else fp4_bulk_copy_g2s(raw_ring + s * FP4_RECORD_BYTES, rec0 + size_t(i) * rec_stride, FP4_RECORD_BYTES, &raw_full[s]);
+        else bulk_copy_g2s(raw_ring + s * FP4_RECORD_BYTES, rec0 + size_t(i) * rec_stride, FP4_RECORD_BYTES, &raw_full[s]);
       };
       auto load_a = [&](int i) {
         const int s = i % A_ST;
@@ -260,24 +217,17 @@ gemm_fp4_grouped_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid
           // the stored byte is code + 6; the fp16 exponent field of 2^(code - 127) is code - 112
           const uint32_t m8 = ((rw & 1) ? (mul >> 8) : (mul & 0xFFu)) - 118u;
           const uint32_t sb = (m8 << 10) | (m8 << 26);
-          *reinterpret_cast<uint4*>(dst + ((j ^ (row & 7)) << 4)) = deq_fp4_word_f16(words[jj], *reinterpret_cast<const __half2*>(&sb));
+          *reinterpret_cast<uint4*>(dst + ((j ^ (row & 7)) << 4)) = deq_fp4_word_f16(words[jj], sb);
         }
       } else {
 #pragma unroll
         for (int jj = 0; jj < WORDS; ++jj) {
           const int j = part * 4 + jj;
           const uint32_t m8 = j < 4 ? (mul & 0xFFu) : (mul >> 8);
-          const uint32_t sb = (m8 << 7) | (m8 << 23);
-          const __nv_bfloat162 s2 = *reinterpret_cast<const __nv_bfloat162*>(&sb);
-          uint4 o;
-          o.x = deq_fp4_pair(words[jj], s2);
-          o.y = deq_fp4_pair(words[jj] >> 4, s2);
-          o.z = deq_fp4_pair(words[jj] >> 8, s2);
-          o.w = deq_fp4_pair(words[jj] >> 12, s2);
-          *reinterpret_cast<uint4*>(dst + ((j ^ (row & 7)) << 4)) = o;
+          *reinterpret_cast<uint4*>(dst + ((j ^ (row & 7)) << 4)) = deq_fp4_word_bf16(words[jj], m8);
         }
       }
-      asm volatile("fence.proxy.async.shared::cta;" ::: "memory");   // generic-proxy stores -> visible to the tensor core
+      fence_proxy_async_smem();   // generic-proxy stores -> visible to the tensor core
       __syncwarp();
       if (lane == 0) {
         mbar_arrive(&deq_full[ws]);
@@ -377,7 +327,7 @@ fp4_stream_grouped_kernel(const void* __restrict__ A_, int lda, const int* __res
           const int nk = min(2, num_kb - 2 * pr);
           mbar_expect_tx(&full[s], uint32_t(nk) * FP4_RECORD_BYTES);
           for (int r = 0; r < nk; ++r)
-            fp4_bulk_copy_g2s(ring + s * FP4_STREAM_STAGE_BYTES + r * FP4_RECORD_BYTES, rec0 + size_t(2 * pr + r) * rec_stride, FP4_RECORD_BYTES,
+            bulk_copy_g2s(ring + s * FP4_STREAM_STAGE_BYTES + r * FP4_RECORD_BYTES, rec0 + size_t(2 * pr + r) * rec_stride, FP4_RECORD_BYTES,
                               &full[s]);
           ++issued;
           if (++s == FP4_STREAM_STAGES) { s = 0; phase ^= 1; }
@@ -543,6 +493,7 @@ static int LaunchFp4Stream(const void* A, int lda, const int* row_map, const uin
 }
 
 bool MakeMapBf16(CUtensorMap* out, const void* ptr, int rows, int cols, int ld, int box_rows);  // gemm_tcgen05.cu
+int LaunchPairFp4(const void* A, int lda, const uint8_t* packed, const GemmParams& p, int token_tile, int max_tiles, bool half, cudaStream_t stream);  // gemm_pair.cu
 bool MakeMapBytes128(CUtensorMap* out, const void* ptr, long long rows, int box_rows);          // gemm_tcgen05.cu
 
 template <int BT, bool HALF, int WBUF, int GROUPS, int NACC>
@@ -641,13 +592,9 @@ OGB_API int ogb_moe_gemm_fp4(const void* A, int lda, const void* Wpacked, void* 
     const int stage_rows = max_rows_per_tile > 0 && max_rows_per_tile < FP4_STREAM_TOKENS ? max_rows_per_tile : FP4_STREAM_TOKENS;
     return LaunchFp4Stream(A, lda, row_map, wp, n_tiles, p, max_tiles, stage_rows, stream);
   }
+  // Tiles of 32 tokens and more run on pairs of SMs (32 experts of 5760 x 2880, us, before -> now: 6000 rows 389 -> 189, 1200 rows 279 -> 136, 400 rows 157 -> 130).
+  if (bt >= 32 && !row_map) return LaunchPairFp4(A, lda, wp, p, bt, max_tiles, half, stream);
   if (row_map) return -6;   // only the streaming kernel reads its rows through a map
-  switch (bt) {
-    case 16: return half ? LaunchFp4<16, true>(ta, tw, w_by_tma, wp, n_tiles, skip, p, grid, stream) : LaunchFp4<16, false>(ta, tw, w_by_tma, wp, n_tiles, skip, p, grid, stream);
-    case 32: return half ? LaunchFp4<32, true>(ta, tw, w_by_tma, wp, n_tiles, skip, p, grid, stream) : LaunchFp4<32, false>(ta, tw, w_by_tma, wp, n_tiles, skip, p, grid, stream);
-    case 64: return half ? LaunchFp4<64, true>(ta, tw, w_by_tma, wp, n_tiles, skip, p, grid, stream) : LaunchFp4<64, false>(ta, tw, w_by_tma, wp, n_tiles, skip, p, grid, stream);
-    case 128: return half ? LaunchFp4<128, true>(ta, tw, w_by_tma, wp, n_tiles, skip, p, grid, stream) : LaunchFp4<128, false>(ta, tw, w_by_tma, wp, n_tiles, skip, p, grid, stream);
-    case 256: return half ? LaunchFp4<256, true>(ta, tw, w_by_tma, wp, n_tiles, skip, p, grid, stream) : LaunchFp4<256, false>(ta, tw, w_by_tma, wp, n_tiles, skip, p, grid, stream);
-  }
+  if (bt == 16) return half ? LaunchFp4<16, true>(ta, tw, w_by_tma, wp, n_tiles, skip, p, grid, stream) : LaunchFp4<16, false>(ta, tw, w_by_tma, wp, n_tiles, skip, p, grid, stream);
   return -5;
 }

@@ -27,10 +27,10 @@
 
 #include "gemm_common.cuh"
 #include "kernels.h"
+#include "packed_weights.cuh"
 
 namespace ogb {
 
-constexpr int W4_RECORD_BYTES = GEMM_BLOCK_N * 32 + GEMM_BLOCK_N * 8;  // 5120
 constexpr int W4_WBUF = 2;                                              // dequantised tiles in flight
 
 template <int BT>
@@ -47,20 +47,6 @@ struct W4Cfg {
   static_assert(RAW >= 4, "raw ring too shallow");
   static_assert(BT * GEMM_BLOCK_N * 4 <= DATA_BYTES, "the parked fp32 tile must fit in the pipeline memory");
 };
-
-__device__ __forceinline__ void bulk_copy_g2s(void* smem_dst, const void* gsrc, uint32_t bytes, uint64_t* bar) {
-  asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
-               ::"r"(smem_u32(smem_dst)), "l"(gsrc), "r"(bytes), "r"(smem_u32(bar)) : "memory");
-}
-__device__ __forceinline__ void fence_proxy_async_smem() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
-
-__device__ __forceinline__ uint32_t deq_pair(uint32_t word, int shift, __nv_bfloat162 z2, __nv_bfloat162 hi2, __nv_bfloat162 lo2) {
-  uint32_t t = ((word >> shift) & 0x000F000Fu) | 0x43004300u;  // two bf16 numbers 128 + q
-  __nv_bfloat162 v = *reinterpret_cast<__nv_bfloat162*>(&t);
-  v = __hsub2(v, z2);
-  v = __hfma2(v, hi2, __hmul2(v, lo2));                          // round((q - zp) * (hi + lo)) in one rounding
-  return *reinterpret_cast<uint32_t*>(&v);
-}
 
 template <int BT>
 __global__ void __launch_bounds__(GEMM_THREADS, W4Cfg<BT>::TWO_PER_SM ? 2 : 1)
@@ -174,19 +160,9 @@ gemm_w4_kernel(const __grid_constant__ CUtensorMap tmap_a, const uint8_t* __rest
       const uint2 sz = *reinterpret_cast<const uint2*>(rec + GEMM_BLOCK_N * 32 + row * 8);
       const uint32_t words[8] = {q0.x, q0.y, q0.z, q0.w, q1.x, q1.y, q1.z, q1.w};
       uint8_t* dst = w_ring + ws * W_TILE_BYTES + row * 128;
+      const W4Scale sc[2] = {w4_scale(sz.x), w4_scale(sz.y)};
 #pragma unroll
-      for (int j = 0; j < 8; ++j) {
-        const uint32_t packed = j < 4 ? sz.x : sz.y;  // (hi, lo | zp) of the 32-block this word belongs to
-        const __nv_bfloat16 hi = __ushort_as_bfloat16(uint16_t(packed & 0xFFFF)), lo = __ushort_as_bfloat16(uint16_t((packed >> 16) & 0xFFF0));
-        const __nv_bfloat16 zp = __ushort_as_bfloat16(uint16_t(0x4300u | ((packed >> 16) & 0xF)));
-        const __nv_bfloat162 hi2 = __halves2bfloat162(hi, hi), lo2 = __halves2bfloat162(lo, lo), z2 = __halves2bfloat162(zp, zp);
-        uint4 o;
-        o.x = deq_pair(words[j], 0, z2, hi2, lo2);
-        o.y = deq_pair(words[j], 4, z2, hi2, lo2);
-        o.z = deq_pair(words[j], 8, z2, hi2, lo2);
-        o.w = deq_pair(words[j], 12, z2, hi2, lo2);
-        *reinterpret_cast<uint4*>(dst + ((j ^ (row & 7)) << 4)) = o;
-      }
+      for (int j = 0; j < 8; ++j) *reinterpret_cast<uint4*>(dst + ((j ^ (row & 7)) << 4)) = deq_w4_word(words[j], sc[j >> 2]);
       fence_proxy_async_smem();   // generic-proxy stores -> visible to the tensor core's async proxy
       mbar_arrive(&deq_full[ws]);
       mbar_arrive(&raw_empty[rs]);
@@ -202,6 +178,8 @@ gemm_w4_kernel(const __grid_constant__ CUtensorMap tmap_a, const uint8_t* __rest
 
 // --------------------------------------------------------------------------------- host side
 bool MakeMapBf16(CUtensorMap* out, const void* ptr, int rows, int cols, int ld, int box_rows);  // gemm_tcgen05.cu
+double PairW4Ns(int M, int N, int total_kb);                                                       // gemm_pair.cu
+int LaunchPairW4(const void* A, int lda, const uint8_t* packed, const GemmParams& p, int force_tiles, cudaStream_t stream);
 
 template <int BT>
 static int LaunchW4(const CUtensorMap& ta, const uint8_t* wp, int n_tiles_total, const GemmParams& p, dim3 grid, cudaStream_t stream) {
@@ -461,6 +439,8 @@ OGB_API int ogb_gemm_w4(const void* A, int lda, const void* Wpacked, void* C, in
       return wide ? LaunchGemvW4<2, 2>(a, lda, w, n_tiles, g, stream) : LaunchGemvW4<2, 1>(a, lda, w, n_tiles, g, stream);
     }
   }
+  const int pair_tiles = splits < 0 ? -splits : 0;      // asks for the paired kernel with that many token tiles
+  const bool auto_split = splits <= 0;
   if (splits <= 0) {
     // Every k-block costs a dequantisation pass on top of the copy, so the k range is cut finer than for bf16 weights:
     // the largest power of two that keeps 8 k-blocks per CTA and all CTAs resident at once.
@@ -476,8 +456,6 @@ OGB_API int ogb_gemm_w4(const void* A, int lda, const void* Wpacked, void* C, in
   if (splits > total_kb) splits = total_kb;
   int kb_per = (total_kb + splits - 1) / splits;
   while (splits > 1 && kb_per * (splits - 1) >= total_kb) { --splits; kb_per = (total_kb + splits - 1) / splits; }
-  CUtensorMap ta;
-  if (!MakeMapBf16(&ta, A, M, K, lda, bt)) return -2;
   GemmParams p = {};
   p.M = M; p.N = N; p.K = K;
   p.splits = splits; p.kb_per_split = kb_per; p.total_kb = total_kb;
@@ -486,8 +464,15 @@ OGB_API int ogb_gemm_w4(const void* A, int lda, const void* Wpacked, void* C, in
   p.bias = static_cast<const __nv_bfloat16*>(bias);
   p.status = status;
   p.pdl = pdl_enabled;
-  dim3 grid(n_tiles, m_tiles, splits);
   const uint8_t* wp = static_cast<const uint8_t*>(Wpacked);
+  // Products of more than 64 tokens run on pairs of SMs unless their few tiles have a long k range, which the split form below divides; a wave of that
+  // form takes about 680 ns per k-block (us, pairs / splits: M 128, N 16384, K 3072 24 / 40; M 128, N 3072, K 8192 45 / 27; M 777, N 3072, K 8192 51 / 96).
+  const double waves = double(((long long)n_tiles * m_tiles * splits + sm_count - 1) / sm_count);
+  if (pair_tiles > 0 || (auto_split && M > 64 && PairW4Ns(M, N, total_kb) < waves * kb_per * 680.0))
+    return LaunchPairW4(A, lda, wp, p, pair_tiles, stream);
+  CUtensorMap ta;
+  if (!MakeMapBf16(&ta, A, M, K, lda, bt)) return -2;
+  dim3 grid(n_tiles, m_tiles, splits);
   switch (bt) {
     case 16: return LaunchW4<16>(ta, wp, n_tiles, p, grid, stream);
     case 32: return LaunchW4<32>(ta, wp, n_tiles, p, grid, stream);
