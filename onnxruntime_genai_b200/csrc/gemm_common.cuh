@@ -117,19 +117,23 @@ struct GemmParams {
 // as two resident CTAs of the shallow form would have, which such a launch never gets).
 template <int BT, bool DEEP = false>
 struct GemmCfg {
+  // k-blocks of a stage: a role's pass over a stage costs 350 cycles and more whatever it holds (300 ns per k-block with one, 155 with two).
+  // Larger tiles have room for three or four stages of one; two stages of two do not cover the latency of the copies (256 tokens: 620 ns per k-block).
+  static constexpr int KB = BT >= 128 ? 1 : 2;
   static constexpr int A_TILE_BYTES = BT * GEMM_BLOCK_K * 2;
-  static constexpr int STAGE_BYTES = W_TILE_BYTES + A_TILE_BYTES;
+  static constexpr int STAGE_BYTES = KB * (W_TILE_BYTES + A_TILE_BYTES);
   // Decode-sized tiles keep two CTAs per SM: more bytes in flight per SM, dynamic balance between
   // SMs, and room for the next kernel's CTAs to become resident and prefetch weights.
   static constexpr bool TWO_PER_SM = BT <= 128 && !DEEP;   // 128-token tiles: two CTAs per SM, one's epilogue under the other's main loop
-  static constexpr int BUDGET = TWO_PER_SM ? 100 * 1024 : 196 * 1024;
-  static constexpr int MAX_STAGES = BUDGET / STAGE_BYTES;
-  static constexpr int STAGES = MAX_STAGES > (DEEP ? 12 : 8) ? (DEEP ? 12 : 8) : MAX_STAGES;
+  static constexpr int BUDGET = TWO_PER_SM ? 110 * 1024 : 200 * 1024;
+  static constexpr int STAGES = BUDGET / STAGE_BYTES;
   static constexpr int TMEM_COLS = BT < 32 ? 32 : BT;
   static constexpr int PARTIAL_BYTES = BT * GEMM_BLOCK_N * 4;  // fp32 tile parked in stage memory
   static constexpr int SSQ_OFFSET = STAGES * STAGE_BYTES + 512;   // per-row sums of squares (folded norm), after the barriers
   static constexpr int SMEM_BYTES = STAGES * STAGE_BYTES + 1024 /*alignment slack*/ + 512 /*barriers*/ + BT * 4;
+  static_assert(STAGES >= 2, "at least two stages");
   static_assert(PARTIAL_BYTES + 16 * 128 * 16 <= STAGES * STAGE_BYTES, "the parked tile and the reduction's staging lines must fit in the pipeline memory");
+  static_assert((TWO_PER_SM ? 2 : 1) * (SMEM_BYTES + 1024) <= 228 * 1024, "shared memory of an SM");
 };
 
 __device__ __forceinline__ uint32_t pack_f16x2(float a, float b) {

@@ -518,10 +518,10 @@ static int DevicePairs() {
   return n;
 }
 
-// How an [M, N] product is cut into token tiles of equal size (a multiple of 32), and its estimated time without the part every launch has: rounds of
-// the pairs x k-blocks x the time of a k-block, which is 1.12 ns per token of the tile down to what a role's pass over a stage takes, and the
-// drain of the last tile.  Measured, us (M 806): N 6144, K 4096 in 4 / 5 / 6 / 7 tiles 41.1 / 36.7 / 35.4 / 46.5 (2 / 2 / 2 / 3 rounds); N 4096, K 14336
-// in 4 / 5 / 8 tiles 80 / 141 / 122 (1 / 2 / 2); one 128 x 256 tile per CTA instead of the pair: 54.1 and 124.5.
+// How an [M, N] product is cut into token tiles of equal size (a multiple of 32), and its estimated time: rounds of the pairs x k-blocks x the time of
+// a k-block, which is 1.12 ns per token of the tile down to what a role's pass over a stage and the copies' latency take, the drain of the last
+// tile and what every launch has.  Measured with weights from HBM, us: M 512, N 28672, K 4096 in 2 / 3 / 4 / 5 tiles 100 / 105 / 121 / 121 (4 / 5 / 7 / 8
+// rounds); M 233, N 6144, K 4096 in 1 / 2 / 3 / 4 tiles 27 / 22 / 20 / 32 (1 / 1 / 1 / 2 rounds); M 512, N 4096, K 14336 in 2 / 4 tiles 76 / 63 (1 round).
 struct PairPlan { int bt, m_tiles; double ns; };
 static PairPlan PlanPair(int M, int N, int total_kb, int pairs, double floor_ns, int force_tiles) {
   const int n_pairs = (N + 255) / 256, least = (M + PAIR_MAX_BT - 1) / PAIR_MAX_BT;
@@ -529,13 +529,13 @@ static PairPlan PlanPair(int M, int N, int total_kb, int pairs, double floor_ns,
   for (int m = force_tiles > 0 ? force_tiles : least; m <= (force_tiles > 0 ? force_tiles : least + 8); ++m) {
     const int bt = min(PAIR_MAX_BT, ((M + m - 1) / m + 31) / 32 * 32), mt = (M + bt - 1) / bt;
     const double rounds = double((n_pairs * mt + pairs - 1) / pairs);
-    const double ns = rounds * total_kb * (1.12 * bt > floor_ns ? 1.12 * bt : floor_ns) + bt / 32 * 400.0;
+    const double ns = rounds * total_kb * (1.12 * bt > floor_ns ? 1.12 * bt : floor_ns) + bt / 32 * 400.0 + 5000.0;
     if (best.bt == 0 || ns < best.ns) best = {bt, mt, ns};
     if (bt == 32) break;
   }
   return best;
 }
-constexpr double PAIR_BF16_FLOOR_NS = 155, PAIR_PACKED_FLOOR_NS = 310;
+constexpr double PAIR_BF16_FLOOR_NS = 200, PAIR_PACKED_FLOOR_NS = 310;
 
 // Estimated times of the paired kernels in ns, to be compared with the other kernels' (gemm_tcgen05.cu, gemm_w4.cu)
 double PairBf16Ns(int M, int N, int total_kb) { return PlanPair(M, N, total_kb, DevicePairs(), PAIR_BF16_FLOOR_NS, 0).ns; }

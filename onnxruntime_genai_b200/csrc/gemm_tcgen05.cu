@@ -7,8 +7,8 @@
 // (256-token tiles, compute bound).  Both operands are K-major in shared memory with the 128-byte
 // swizzle written by TMA; accumulators live in tensor memory and are read back with tcgen05.ld.
 //
-// Warp roles (192 threads): warp 0 = TMA producer (one lane), warp 1 = MMA issuer (one lane),
-// warps 2..5 = epilogue (warp 2 also owns the TMEM allocation).
+// Warp roles (192 threads): warp 0 = TMA producer, warp 1 = MMA issuer, both as whole warps with one elected lane,
+// warps 2..5 = epilogue (warp 2 also owns the TMEM allocation).  A pipeline stage holds two k-blocks of 64 (see GemmCfg).
 //
 // Split-K (decode: N/128 tiles alone cannot fill 148 SMs) runs as a thread-block CLUSTER of up to
 // 8 CTAs along z: each CTA accumulates its K slice in its own tensor memory and parks the fp32 tile
@@ -51,7 +51,7 @@ template <int BT, int COMM, bool DEEP>
 __global__ void __launch_bounds__(GEMM_THREADS, GemmCfg<BT, DEEP>::TWO_PER_SM ? 2 : 1)
 gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant__ CUtensorMap tmap_a, const GemmParams p) {
   using Cfg = GemmCfg<BT, DEEP>;
-  constexpr int STAGES = Cfg::STAGES;
+  constexpr int STAGES = Cfg::STAGES, KB = Cfg::KB;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   uint64_t* full_bar = reinterpret_cast<uint64_t*>(smem + STAGES * Cfg::STAGE_BYTES);
@@ -62,13 +62,13 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_con
   volatile uint32_t* use_slot = reinterpret_cast<volatile uint32_t*>(tmem_slot + 2);
   float* ssq = reinterpret_cast<float*>(smem + Cfg::SSQ_OFFSET);   // [BT] sums of squares of the activation rows (folded norm)
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = __shfl_sync(0xffffffffu, int(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;
   const int n_tile = blockIdx.x, split = blockIdx.z;
   const int batch = p.bat.m_tiles > 0 ? blockIdx.y / p.bat.m_tiles : 0;        // problem of a batched launch
   const int m_tile = blockIdx.y - batch * p.bat.m_tiles;
   const int a_col0 = batch * p.bat.a_cols;
   const int kb0 = split * p.kb_per_split;
-  const int num_kb = min(p.kb_per_split, p.total_kb - kb0);
+  const int num_kb = min(p.kb_per_split, p.total_kb - kb0), num_st = (num_kb + KB - 1) / KB;      // (the last stage may hold fewer k-blocks)
   // Grouped mode: the tile list is written by the kernel before this one, so nothing is read ahead of it.
   const bool grouped = p.grp.tile_expert != nullptr;
   int row0 = m_tile * BT, rows = min(BT, p.M - row0), w_row0 = batch * p.N;
@@ -102,63 +102,80 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_con
   const uint32_t tmem_base = *tmem_slot;
   if (p.pdl) pdl_launch_dependents();
 
-  auto stage_w = [&](int s) { return smem + s * Cfg::STAGE_BYTES; };
-  auto stage_a = [&](int s) { return smem + s * Cfg::STAGE_BYTES + W_TILE_BYTES; };
+  auto stage_w = [&](int s) { return smem + s * Cfg::STAGE_BYTES; };                              // [KB] weight tiles, [KB] activation tiles
+  auto stage_a = [&](int s) { return smem + s * Cfg::STAGE_BYTES + KB * W_TILE_BYTES; };
+  auto blocks_of = [&](int i) { return min(KB, num_kb - i * KB); };                                // k-blocks of stage i
   auto fail = [&](int code) { atomicMax(p.status, code); *abort_flag = 1; };
 
   if (warp == 0) {
-    if (lane == 0) {
-      // ------------------------------------------------------------------ TMA producer
-      auto load_w = [&](int i) {
-        const int s = i % STAGES;
-        mbar_expect_tx(&full_bar[s], gather ? W_TILE_BYTES : Cfg::STAGE_BYTES);
-        tma_load_2d(stage_w(s), &tmap_w, &full_bar[s], (kb0 + i) * GEMM_BLOCK_K, w_row0 + n_tile * GEMM_BLOCK_N);
-      };
-      auto load_a = [&](int i) {
-        if (gather) return;   // assembled by warps 2..5 below
-        tma_load_2d(stage_a(i % STAGES), &tmap_a, &full_bar[i % STAGES], a_col0 + (kb0 + i) * GEMM_BLOCK_K, row0);
-      };
-      // Weights are never written by an earlier kernel of the stream: fill the pipeline with them
-      // before waiting for the producer of the activations.
-      const int pre = min(STAGES, num_kb);
-      for (int i = 0; i < pre; ++i) load_w(i);
-      if (p.pdl) pdl_wait();
-      if (COMM != 0) *use_slot = comm_open_call(p.comm, gridDim.x * gridDim.y * gridDim.z);
-      for (int i = 0; i < pre; ++i) load_a(i);
-      int issued = pre;
-      for (int i = pre; i < num_kb; ++i) {
-        const int s = i % STAGES;
-        const uint32_t ph = (i / STAGES) & 1;
-        if (!mbar_wait_bounded(&empty_bar[s], ph ^ 1, abort_flag)) { fail(OGB_ERR_WAIT_TMA); break; }
-        load_w(i);
-        load_a(i);
-        ++issued;
+    // ------------------------------------------------------------------ TMA producer
+    auto load_w = [&](int i, int s) {
+      if (elect_one()) {
+        const int nk = blocks_of(i), k0 = (kb0 + i * KB) * GEMM_BLOCK_K;
+        mbar_expect_tx(&full_bar[s], uint32_t(nk) * (gather ? W_TILE_BYTES : W_TILE_BYTES + Cfg::A_TILE_BYTES));
+#pragma unroll
+        for (int h = 0; h < KB; ++h)
+          if (h < nk) tma_load_2d(stage_w(s) + h * W_TILE_BYTES, &tmap_w, &full_bar[s], k0 + h * GEMM_BLOCK_K, w_row0 + n_tile * GEMM_BLOCK_N);
       }
-      if (*abort_flag) {
-        // Copies already issued still write this CTA's shared memory: give them time to land.
-        volatile int never = 0;
-        for (int i = max(0, issued - STAGES); i < issued; ++i)
-          mbar_wait_bounded(&full_bar[i % STAGES], (i / STAGES) & 1, &never, 200000000ull);
+      __syncwarp();
+    };
+    auto load_a = [&](int i, int s) {
+      if (gather) return;   // assembled by warps 2..5 below
+      if (elect_one()) {
+        const int nk = blocks_of(i), k0 = a_col0 + (kb0 + i * KB) * GEMM_BLOCK_K;
+#pragma unroll
+        for (int h = 0; h < KB; ++h)
+          if (h < nk) tma_load_2d(stage_a(s) + h * Cfg::A_TILE_BYTES, &tmap_a, &full_bar[s], k0 + h * GEMM_BLOCK_K, row0);
       }
+      __syncwarp();
+    };
+    // Weights are never written by an earlier kernel of the stream: fill the pipeline with them
+    // before waiting for the producer of the activations.
+    const int pre = min(STAGES, num_st);
+    for (int i = 0; i < pre; ++i) load_w(i, i);
+    if (p.pdl) pdl_wait();
+    if (COMM != 0 && lane == 0) *use_slot = comm_open_call(p.comm, gridDim.x * gridDim.y * gridDim.z);
+    __syncwarp();
+    for (int i = 0; i < pre; ++i) load_a(i, i);
+    int issued = pre, s = 0;
+    uint32_t ph = 0;
+    for (int i = pre; i < num_st; ++i) {
+      if (!__all_sync(0xffffffffu, mbar_wait_bounded(&empty_bar[s], ph, abort_flag))) { fail(OGB_ERR_WAIT_TMA); break; }
+      load_w(i, s);
+      load_a(i, s);
+      ++issued;
+      if (++s == STAGES) { s = 0; ph ^= 1; }
+    }
+    if (*abort_flag) {
+      // Copies already issued still write this CTA's shared memory: give them time to land.
+      volatile int never = 0;
+      for (int i = max(0, issued - STAGES); i < issued; ++i)
+        mbar_wait_bounded(&full_bar[i % STAGES], (i / STAGES) & 1, &never, 200000000ull);
     }
   } else if (warp == 1) {
-    if (lane == 0) {
-      // ------------------------------------------------------------------ MMA issuer
-      constexpr uint32_t idesc = umma_idesc_f16(GEMM_BLOCK_N, BT, 1);
-      bool ok = true;
-      for (int i = 0; i < num_kb && ok; ++i) {
-        const int s = i % STAGES;
-        const uint32_t ph = (i / STAGES) & 1;
-        if (!mbar_wait_bounded(&full_bar[s], ph, abort_flag)) { fail(OGB_ERR_WAIT_TMA); ok = false; break; }
-        tc_fence_after();
-        const uint32_t w = smem_u32(stage_w(s)), a = smem_u32(stage_a(s));
+    // ------------------------------------------------------------------ MMA issuer
+    constexpr uint32_t idesc = umma_idesc_f16(GEMM_BLOCK_N, BT, 1);
+    int s = 0;
+    uint32_t ph = 0;
+    for (int i = 0; i < num_st; ++i) {
+      if (!__all_sync(0xffffffffu, mbar_wait_bounded(&full_bar[s], ph, abort_flag))) { fail(OGB_ERR_WAIT_TMA); break; }
+      tc_fence_after();
+      if (elect_one()) {
+        const uint64_t dw = umma_desc_sw128(smem_u32(stage_w(s))), da = umma_desc_sw128(smem_u32(stage_a(s)));
+        const int nk = blocks_of(i);
 #pragma unroll
-        for (int k = 0; k < GEMM_BLOCK_K / GEMM_UMMA_K; ++k)
-          umma_f16(tmem_base, umma_desc_sw128(w + k * GEMM_UMMA_K * 2), umma_desc_sw128(a + k * GEMM_UMMA_K * 2), idesc,
-                   (i > 0 || k > 0) ? 1u : 0u);
+        for (int h = 0; h < KB; ++h) {
+          if (h >= nk) break;
+#pragma unroll
+          for (int k = 0; k < GEMM_BLOCK_K / GEMM_UMMA_K; ++k)
+            umma_f16(tmem_base, dw + (h * W_TILE_BYTES + k * GEMM_UMMA_K * 2) / 16, da + (h * Cfg::A_TILE_BYTES + k * GEMM_UMMA_K * 2) / 16, idesc,
+                     (i > 0 || h > 0 || k > 0) ? 1u : 0u);
+        }
         umma_commit(&empty_bar[s]);
+        if (i == num_st - 1) umma_commit(accum_bar);
       }
-      if (ok) umma_commit(accum_bar);
+      __syncwarp();
+      if (++s == STAGES) { s = 0; ph ^= 1; }
     }
   }
 
@@ -174,22 +191,24 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_con
     const size_t plane_lines = size_t(p.comm.plane_elems) / 4;
     const uint4* base = p.comm.buf[p.comm.rank] + size_t(ep & 1) * p.comm.world * plane_lines;
     bool dead = *reinterpret_cast<volatile int*>(p.status) != 0;
-    for (int i = 0; i < num_kb; ++i) {
+    for (int i = 0; i < num_st; ++i) {
       const int s = i % STAGES;
       if (i >= STAGES && !mbar_wait_bounded(&empty_bar[s], ((i / STAGES) & 1) ^ 1, abort_flag)) { fail(OGB_ERR_WAIT_TMA); }
-      uint8_t* tile = stage_a(s);
-      const int k0 = (kb0 + i) * GEMM_BLOCK_K;
-      for (int idx = gt; idx < BT * 16; idx += 128) {
-        const int r = idx >> 4, ln = idx & 15;          // row of the tile, line of the row (4 bf16 each)
-        const int m = row0 + r, k = k0 + ln * 4;
-        uint2 d = make_uint2(0u, 0u);
-        if (r < rows && k < p.K) {
-          const int owner = m / p.ag_rows, rl = m - owner * p.ag_rows;
-          const uint4 q = wait_line(base + size_t(owner) * plane_lines + (size_t(rl) * p.K + k) / 4, flag, dead, p.status);
-          d = make_uint2(q.x, q.z);
+      for (int h = 0; h < blocks_of(i); ++h) {
+        uint8_t* tile = stage_a(s) + h * Cfg::A_TILE_BYTES;
+        const int k0 = (kb0 + i * KB + h) * GEMM_BLOCK_K;
+        for (int idx = gt; idx < BT * 16; idx += 128) {
+          const int r = idx >> 4, ln = idx & 15;          // row of the tile, line of the row (4 bf16 each)
+          const int m = row0 + r, k = k0 + ln * 4;
+          uint2 d = make_uint2(0u, 0u);
+          if (r < rows && k < p.K) {
+            const int owner = m / p.ag_rows, rl = m - owner * p.ag_rows;
+            const uint4 q = wait_line(base + size_t(owner) * plane_lines + (size_t(rl) * p.K + k) / 4, flag, dead, p.status);
+            d = make_uint2(q.x, q.z);
+          }
+          const int chunk = ln >> 1;
+          *reinterpret_cast<uint2*>(tile + r * 128 + (((chunk ^ (r & 7)) << 4) | ((ln & 1) << 3))) = d;
         }
-        const int chunk = ln >> 1;
-        *reinterpret_cast<uint2*>(tile + r * 128 + (((chunk ^ (r & 7)) << 4) | ((ln & 1) << 3))) = d;
       }
       asm volatile("fence.proxy.async.shared::cta;" ::: "memory");   // generic-proxy writes -> visible to tcgen05.mma
       mbar_arrive(&full_bar[s]);
@@ -207,17 +226,21 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_con
     float acc[PER];
 #pragma unroll
     for (int k = 0; k < PER; ++k) acc[k] = 0.f;
-    for (int i = 0; i < num_kb; ++i) {
+    for (int i = 0; i < num_st; ++i) {
       const int s = i % STAGES;
       if (!mbar_wait_bounded(&full_bar[s], (i / STAGES) & 1, abort_flag)) { fail(OGB_ERR_WAIT_TMA); break; }
-      const uint8_t* tile = stage_a(s);
 #pragma unroll
-      for (int k = 0; k < PER; ++k) {
-        const int c = t + 128 * k;
-        if (c < CHUNKS) {
-          const uint4 q = *reinterpret_cast<const uint4*>(tile + c * 16);
-          const float2 a = unpack_bf16x2(q.x), b = unpack_bf16x2(q.y), cc = unpack_bf16x2(q.z), d = unpack_bf16x2(q.w);
-          acc[k] += a.x * a.x + a.y * a.y + b.x * b.x + b.y * b.y + cc.x * cc.x + cc.y * cc.y + d.x * d.x + d.y * d.y;
+      for (int h = 0; h < KB; ++h) {
+        if (h >= blocks_of(i)) break;
+        const uint8_t* tile = stage_a(s) + h * Cfg::A_TILE_BYTES;
+#pragma unroll
+        for (int k = 0; k < PER; ++k) {
+          const int c = t + 128 * k;
+          if (c < CHUNKS) {
+            const uint4 q = *reinterpret_cast<const uint4*>(tile + c * 16);
+            const float2 a = unpack_bf16x2(q.x), b = unpack_bf16x2(q.y), cc = unpack_bf16x2(q.z), d = unpack_bf16x2(q.w);
+            acc[k] += a.x * a.x + a.y * a.y + b.x * b.x + b.y * b.y + cc.x * cc.x + cc.y * cc.y + d.x * d.x + d.y * d.y;
+          }
         }
       }
       __syncwarp();
@@ -433,6 +456,7 @@ OGB_API int ogb_gemm_auto_splits(int M, int N, int K, int dual, int sm_count) {
     const int kbs = total_kb / s;
     // 8 partitions: long k ranges whose 4-way split would not fit one CTA per SM (that form runs the deep pipeline: down
     // 25.1 us at s=4 against 27.7 at s=8), or launches so small that even 8 partitions leave one CTA per SM
+    if (s == 8 && bt == 256) break;       // (eight CTAs of a cluster at one per SM: a second wave, N 2048, K 8192 40 us against 26 with four)
     const bool ok = s <= 4 ? kbs >= 2 : ((kbs >= 16 && tiles * 4 > sm_count) || (tiles * s <= sm_count && kbs >= 8));
     if (ok) best = s;
   }
@@ -619,11 +643,14 @@ OGB_API int ogb_gemm_bf16_fused(const void* A, int lda, const void* W, int ldw, 
     p.rope.Hq = f->Hq; p.rope.Hkv = f->Hkv; p.rope.D = f->D; p.rope.rot = f->rot; p.rope.max_pos = f->max_pos;
     extras = true;
   }
-  // Prompt-sized products run on pairs of SMs.  The (tiles x k-splits) form below keeps those of up to 256 tokens whose tiles leave pairs idle over a
-  // long k range; a wave of it takes about 310 ns per k-block (M 233, N 4096, us, pairs / splits: K 4096 17 / 21, K 14336 60 / 40).
-  if (!extras && !p.comm_epilogue && p.ag_rows == 0) {
-    const double waves = double(((long long)n_tiles * m_tiles * splits + sm_count - 1) / sm_count);
-    if (pair_tiles > 0 || (auto_split && bt == 256 && (M > 256 || PairBf16Ns(M, N, total_kb) < waves * kb_per * 310.0)))
+  // Prompt-sized products run on pairs of SMs.  The (tiles x k-splits) form below keeps those whose few tiles leave pairs idle over a long k range; its
+  // CTAs take about 420 ns per k-block (128-token tiles: 470, two CTAs per SM) and 10 us beside.  Weights from HBM, us, pairs / splits: M 233, N 4096, K 4096
+  // 19 / 21, K 14336 56 / 39; M 80, N 4096, K 14336 54 / 35; M 80, N 16384, K 2048 16 / 23; M 200, N 4096, K 960 8 / 15.  Short k ranges stay here although
+  // pairs are faster (K 512 5 / 13): the gathered form of a product, which only this kernel has, gives the same bits as the plain one.
+  if (!extras && !p.comm_epilogue && p.ag_rows == 0 && (pair_tiles > 0 || (auto_split && M > 64 && (M > 256 || total_kb > 8)))) {
+    const double slots = bt == 128 ? 2.0 * sm_count : 1.0 * sm_count, ctas = double(n_tiles) * m_tiles * splits;
+    const double waves = double((long long)((ctas + slots - 1) / slots));
+    if (pair_tiles > 0 || PairBf16Ns(M, N, total_kb) < waves * kb_per * (bt == 128 ? 470.0 : 420.0) + 10000.0)
       return LaunchPairBf16(A, lda, W, ldw, p, pair_tiles, stream);
   }
   dim3 grid(n_tiles, m_tiles, splits);

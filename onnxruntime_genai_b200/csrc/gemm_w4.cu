@@ -466,9 +466,9 @@ OGB_API int ogb_gemm_w4(const void* A, int lda, const void* Wpacked, void* C, in
   p.pdl = pdl_enabled;
   const uint8_t* wp = static_cast<const uint8_t*>(Wpacked);
   // Products of more than 64 tokens run on pairs of SMs unless their few tiles have a long k range, which the split form below divides; a wave of that
-  // form takes about 680 ns per k-block (us, pairs / splits: M 128, N 16384, K 3072 24 / 40; M 128, N 3072, K 8192 45 / 27; M 777, N 3072, K 8192 51 / 96).
+  // form takes about 680 ns per k-block and 6 us beside (us, pairs / splits: M 128, N 16384, K 3072 24 / 40; M 128, N 3072, K 8192 45 / 27; M 777, N 3072, K 8192 51 / 96).
   const double waves = double(((long long)n_tiles * m_tiles * splits + sm_count - 1) / sm_count);
-  if (pair_tiles > 0 || (auto_split && M > 64 && PairW4Ns(M, N, total_kb) < waves * kb_per * 680.0))
+  if (pair_tiles > 0 || (auto_split && M > 64 && PairW4Ns(M, N, total_kb) < waves * kb_per * 680.0 + 6000.0))
     return LaunchPairW4(A, lda, wp, p, pair_tiles, stream);
   CUtensorMap ta;
   if (!MakeMapBf16(&ta, A, M, K, lda, bt)) return -2;
