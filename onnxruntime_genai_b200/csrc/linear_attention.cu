@@ -7,9 +7,9 @@
 //   gated_delta_kernel        decode-shaped steps.  One CTA = (request, value head, 32 columns of the head's state S [dk, dv]); a thread
 //                             keeps 16 to 64 rows of one column, the lanes of a warp are neighbouring columns (the state streams in
 //                             full lines), the row splits of a column meet in shared memory.
-//   gated_delta_chunk_kernel  prompts.  The row splits of a column are lanes of one warp, so that the two dot products of a token are
-//                             finished by shuffles and the token loop has no barrier; the keys and queries of a chunk of tokens
-//                             are normalised into shared memory by all warps beforehand.
+//   gated_delta_chunk_kernel  prompts.  Tokens four at a time; the row splits of a column are lanes of one warp, so that dot products are
+//                             finished by shuffles and the loop over blocks has no barrier; the keys and queries of a chunk of tokens
+//                             are normalised into shared memory; lengths, gates and the products within a block come from gdn_prepare_kernel.
 // Per token, with k_t, q_t of the head:
 //     S[:, j] *= exp(g);   mem = sum_i S[i, j] k[i];   delta = (v[j] - mem) * beta;   S[i, j] += k[i] * delta;   o[j] = sum_i S[i, j] q[i]
 // Tokens of a request are walked in order inside the kernel (a decode step is one token, a prompt chunk many); the state is read
@@ -146,30 +146,124 @@ __global__ void __launch_bounds__(512) gated_delta_kernel(GdnParams<T> p) {
   }
 }
 
-// A thread owns two columns and NPT rows of each, 8 * NPT >= dk; the lanes of a warp are 4 column pairs x 8 row splits.  Row of split sp,
-// register i: (i / 4) * 32 + sp * 4 + i % 4, so that a thread's rows come as groups of four and the splits of a warp read one
-// 128-byte line of a key together.  CH tokens per chunk.
-// Both dot products of a token are taken on the state before its update, which needs the two vectors once and one round of
-// shuffles: with m = S^T k and r = S^T q (old state), delta = beta * (v - g m), S <- g S + k delta^T and S_new^T q = g r + (k . q) delta.
+// What the chunk kernel needs of a block of four tokens beside their rows, per value head: E_st (k_s . k_t) for (s, t) = (0,1) (0,2) (1,2) (0,3) (1,3)
+// (2,3) at 0 .. 5; E_st (k_s . q_t) at 8 + 4 t + s, s <= t; D_t at 24; E_t3 at 28; beta_t at 32 (names below).  Tokens past a request's end:
+// keys, values and beta zero, decay one.  Blocks of request r are numbered from cu_seqlens[r] / 4 + r on.
+constexpr int GDN_BLOCK = 4, GDN_COEF = 40;
+__host__ __device__ inline long long gdn_blocks(long long T, long long B) { return T / GDN_BLOCK + B; }
+
+// One warp per block and value head: lengths of the block's keys and queries (`lengths` [T, Hk]: the factors that make them unit vectors)
+// and its coefficients.
+template <typename T>
+__global__ void __launch_bounds__(256) gdn_prepare_kernel(GdnParams<T> p, int B, float2* __restrict__ lengths, float* __restrict__ coef) {
+  pdl_launch_dependents();
+  pdl_wait();
+  const int lane = threadIdx.x & 31, h = blockIdx.y * 8 + (threadIdx.x >> 5), id = blockIdx.x;
+  if (h >= p.Hv) return;
+  int lo = 0, hi = B - 1;                                  // the request: last r with its first block <= id
+  while (lo < hi) {
+    const int mid = (lo + hi + 1) >> 1;
+    if (p.cu_seqlens[mid] / GDN_BLOCK + mid <= id) lo = mid; else hi = mid - 1;
+  }
+  const int t0 = p.cu_seqlens[lo] + (id - p.cu_seqlens[lo] / GDN_BLOCK - lo) * GDN_BLOCK, n = min(GDN_BLOCK, p.cu_seqlens[lo + 1] - t0);
+  if (n <= 0) return;
+  const int dk = p.dk, rep = p.Hv / p.Hk, hk = h / rep;
+  float val[16], len[8];
+#pragma unroll
+  for (int i = 0; i < 16; ++i) val[i] = 0.f;
+#pragma unroll
+  for (int i = 0; i < 8; ++i) len[i] = 0.f;
+  for (int i = lane; i < dk; i += 32) {
+    float k[4], q[4];
+#pragma unroll
+    for (int t = 0; t < 4; ++t) {
+      const size_t at = size_t(t0 + t) * p.tok_stride_qk + size_t(hk) * dk + i;
+      k[t] = t < n ? act_f32(p.k[at]) : 0.f;
+      q[t] = t < n ? act_f32(p.q[at]) : 0.f;
+      len[t] = fmaf(k[t], k[t], len[t]);
+      len[4 + t] = fmaf(q[t], q[t], len[4 + t]);
+    }
+    int j = 0;
+#pragma unroll
+    for (int t = 1; t < 4; ++t)
+#pragma unroll
+      for (int s = 0; s < t; ++s, ++j) val[j] = fmaf(k[s], k[t], val[j]);
+#pragma unroll
+    for (int t = 0; t < 4; ++t)
+#pragma unroll
+      for (int s = 0; s <= t; ++s, ++j) val[j] = fmaf(k[s], q[t], val[j]);
+  }
+#pragma unroll
+  for (int i = 0; i < 8; ++i) {
+    len[i] = p.l2norm ? inv_length(warp_sum(len[i]), p.l2_eps) : 1.f;
+    if (p.l2norm && i >= 4) len[i] *= p.q_scale;
+  }
+#pragma unroll
+  for (int o = 8; o > 0; o >>= 1) {
+    const bool up = (lane & o) != 0;
+#pragma unroll
+    for (int i = 0; i < o; ++i) {
+      const float send = up ? val[i] : val[i + o], keep = up ? val[i + o] : val[i];
+      val[i] = keep + __shfl_xor_sync(0xffffffffu, send, o);
+    }
+  }
+  const float dot = val[0] + __shfl_xor_sync(0xffffffffu, val[0], 16);       // sum number lane % 16
+  float decay = 1.f, beta = 0.f;
+  if (lane < n) gdn_gates(p, t0 + lane, h, decay, beta);
+  float g[4];
+#pragma unroll
+  for (int u = 0; u < 4; ++u) g[u] = __shfl_sync(0xffffffffu, decay, u);
+  beta = __shfl_sync(0xffffffffu, beta, lane & 3);
+  const int pr = lane & 15;
+  const bool kq = pr >= 6;
+  int t = kq ? 0 : 1, s = kq ? pr - 6 : pr;
+  while (s >= t + (kq ? 1 : 0)) { s -= t + (kq ? 1 : 0); ++t; }
+  auto pick = [&](int base, int i) { return i == 0 ? len[base] : i == 1 ? len[base + 1] : i == 2 ? len[base + 2] : len[base + 3]; };
+  auto span = [&](int from, int to) {                      // decays of tokens from .. to
+    float e = 1.f;
+#pragma unroll
+    for (int u = 0; u < 4; ++u) e *= u >= from && u <= to ? g[u] : 1.f;
+    return e;
+  };
+  float* c = coef + (size_t(id) * p.Hv + h) * GDN_COEF;
+  if (lane < 16) c[kq ? 8 + 4 * t + s : pr] = dot * pick(0, s) * (kq ? pick(4, t) : pick(0, t)) * span(s + 1, t);
+  else if (lane < 20) c[24 + (lane & 3)] = span(0, lane & 3);
+  else if (lane < 24) c[28 + (lane & 3)] = span((lane & 3) + 1, 3);
+  else if (lane < 28) c[32 + (lane & 3)] = beta;
+  if (h == hk * rep && lane < n) lengths[size_t(t0 + lane) * p.Hk + hk] = make_float2(pick(0, lane), pick(4, lane));
+}
+
+// A thread owns two columns and NPT rows of each, 16 * NPT >= dk; the lanes of a warp are 2 column pairs x 16 row splits.  Row of split sp,
+// register i: (i / 4) * 64 + sp * 4 + i % 4, so that a thread's rows come as groups of four and the splits of a warp read two
+// 128-byte lines of a key together.  CH tokens per chunk, walked in blocks of four.
+// With one token at a time the kernel is a chain of latencies (dot products, shuffles, the update: 980 cycles a token).  The tokens of a block
+// therefore meet the state S before the block, m_t = S^T k_t and r_t = S^T q_t, eight dot products at once, and the block's own part is put right
+// with the dot products of its keys and queries, which do not depend on the state (gdn_prepare_kernel).  With the decays g_t,
+// D_t = g_0 .. g_t and E_st = g_(s+1) .. g_t:
+//     delta_t = beta_t (v_t - D_t m_t - sum_(s<t) E_st (k_s . k_t) delta_s)
+//     o_t = D_t r_t + sum_(s<=t) E_st (k_s . q_t) delta_s            S <- D_3 S + sum_s E_s3 k_s delta_s^T
+// The sixteen sums of a column pair are reduced over its lanes by halving (8 + 4 + 2 + 1 shuffles, lane j ends with sum j).
+// 3001 tokens, 16 heads of 128 x 128: 1535 us with one token at a time, 1202 with all of this inside the kernel, 766 + 19 (prepare).
+// vec: rows of keys and queries start on 16 bytes and dk is a multiple of 8.
 template <typename T, int NPT, int CH>
-__global__ void __launch_bounds__(128) gated_delta_chunk_kernel(GdnParams<T> p) {
-  constexpr int DKP = NPT * 8, G4 = NPT / 4;
+__global__ void __launch_bounds__(128) gated_delta_chunk_kernel(GdnParams<T> p, const float2* __restrict__ lengths, const float* __restrict__ coef, int vec) {
+  constexpr int DKP = NPT * 16, G4 = NPT / 4, LD = DKP + 4, BLK = GDN_BLOCK, NB = CH / BLK, COLS = 16;
   pdl_launch_dependents();
   pdl_wait();
   const int b = blockIdx.x, h = blockIdx.y;
   const int Hv = p.Hv, dv = p.dv, dk = p.dk;
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, sp = lane & 7;
-  const int jj = warp * 8 + (lane >> 3) * 2, j = blockIdx.z * 32 + jj;      // columns j, j + 1
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, sp = lane & 15;
+  const int jj = warp * 4 + (lane >> 4) * 2, j = blockIdx.z * COLS + jj;      // columns j, j + 1
   const int hk = h / (Hv / p.Hk);
   const int t0 = p.cu_seqlens[b], t1 = p.cu_seqlens[b + 1];
   if (t0 >= t1) return;
-  __shared__ __align__(16) float sk[CH][DKP];
-  __shared__ __align__(16) float sq[CH][DKP];
-  __shared__ __align__(8) float sv[CH][32];
-  __shared__ float sdot[CH], sgate[2][CH];
+  __shared__ __align__(16) float sk[CH][LD];
+  __shared__ __align__(16) float sq[CH][LD];
+  __shared__ __align__(8) float sv[CH][COLS];
+  __shared__ __align__(16) float scoef[NB][GDN_COEF];
   const bool live0 = j < dv, live1 = j + 1 < dv, fresh = p.past_lens[b] == 0;
   float* S = p.state + size_t(p.slots[b]) * p.slot_stride + size_t(h) * dk * dv;
-  auto row_of = [&](int i) { return (i >> 2) * 32 + sp * 4 + (i & 3); };
+  auto row_of = [&](int i) { return (i >> 2) * 64 + sp * 4 + (i & 3); };
   float c0[NPT], c1[NPT];
 #pragma unroll
   for (int i = 0; i < NPT; ++i) {
@@ -179,97 +273,130 @@ __global__ void __launch_bounds__(128) gated_delta_chunk_kernel(GdnParams<T> p) 
   }
 
   // a chunk's raw keys / queries / values on their way from global memory: held in registers while the previous chunk is computed
-  constexpr int PER = DKP / 32, TW = CH / 4;               // elements per lane of a row, rows per warp
+  constexpr int VEC = DKP / 8, U = CH * VEC / 128;         // groups of eight columns of a row; groups of keys (and of queries) per thread
+  static_assert(U * 128 == CH * VEC && NB * (GDN_COEF / 4) <= 128, "whole passes");
   const T zero = act_from<T>(0.f);
-  T rk[TW][PER], rq[TW][PER], rv[TW];
-  float ga, gb;
+  const int first_block = t0 / BLK + b;
+  struct alignas(16) Eight { T v[8]; };
+  Eight raw[2 * U];
+  float2 len[U];
+  T rv[CH * COLS / 128];
+  float4 rc;
   auto fetch = [&](int f0) {
 #pragma unroll
-    for (int w = 0; w < TW; ++w) {
-      const int t = f0 + w * 4 + warp;
+    for (int u = 0; u < U; ++u) {
+      const int idx = threadIdx.x + 128 * u, t = f0 + idx / VEC, c = (idx % VEC) * 8;
+      const bool in = t < t1;
+      len[u] = in ? lengths[size_t(t) * p.Hk + hk] : make_float2(0.f, 0.f);
+      const size_t at = size_t(in ? t : t0) * p.tok_stride_qk + size_t(hk) * dk + c;
+      if (vec && in && c < dk) {
+        raw[u] = *reinterpret_cast<const Eight*>(p.k + at);
+        raw[U + u] = *reinterpret_cast<const Eight*>(p.q + at);
+      } else {
 #pragma unroll
-      for (int e = 0; e < PER; ++e) {
-        const int i = e * 32 + lane;
-        const bool ok = t < t1 && i < dk;
-        rk[w][e] = ok ? p.k[size_t(t) * p.tok_stride_qk + size_t(hk) * dk + i] : zero;
-        rq[w][e] = ok ? p.q[size_t(t) * p.tok_stride_qk + size_t(hk) * dk + i] : zero;
+        for (int e = 0; e < 8; ++e) {
+          const bool ok = in && c + e < dk;
+          raw[u].v[e] = ok ? p.k[at + e] : zero;
+          raw[U + u].v[e] = ok ? p.q[at + e] : zero;
+        }
       }
-      const int jc = blockIdx.z * 32 + lane;
-      rv[w] = (t < t1 && jc < dv) ? p.v[size_t(t) * p.tok_stride_v + size_t(h) * dv + jc] : zero;
     }
-    ga = gb = 0.f;
-    if (threadIdx.x < CH && f0 + int(threadIdx.x) < t1) gdn_gates(p, f0 + threadIdx.x, h, ga, gb);
+#pragma unroll
+    for (int u = 0; u < CH * COLS / 128; ++u) {
+      const int idx = threadIdx.x + 128 * u, t = f0 + idx / COLS, c = blockIdx.z * COLS + idx % COLS;
+      rv[u] = t < t1 && c < dv ? p.v[size_t(t) * p.tok_stride_v + size_t(h) * dv + c] : zero;
+    }
+    const int blk = threadIdx.x / (GDN_COEF / 4);
+    if (blk < NB && f0 + blk * BLK < t1)
+      rc = reinterpret_cast<const float4*>(coef + (size_t(first_block + (f0 - t0) / BLK + blk) * Hv + h) * GDN_COEF)[threadIdx.x % (GDN_COEF / 4)];
   };
   fetch(t0);
   for (int f0 = t0; f0 < t1; f0 += CH) {
     __syncthreads();                                       // the previous chunk is no longer read
 #pragma unroll
-    for (int w = 0; w < TW; ++w) {
-      float ssk = 0.f, ssq = 0.f, skq = 0.f;
-#pragma unroll
-      for (int e = 0; e < PER; ++e) {
-        const float kk = act_f32(rk[w][e]), qq = act_f32(rq[w][e]);
-        ssk += kk * kk; ssq += qq * qq; skq += kk * qq;
-      }
-      float nk = 1.f, nq = 1.f;
-      if (p.l2norm) {
-        nk = inv_length(warp_sum(ssk), p.l2_eps);
-        nq = p.q_scale * inv_length(warp_sum(ssq), p.l2_eps);
-      }
-      skq = warp_sum(skq) * nk * nq;
-      const int tt = w * 4 + warp;
-#pragma unroll
-      for (int e = 0; e < PER; ++e) {
-        sk[tt][e * 32 + lane] = act_f32(rk[w][e]) * nk;
-        sq[tt][e * 32 + lane] = act_f32(rq[w][e]) * nq;
-      }
-      sv[tt][lane] = act_f32(rv[w]);
-      if (lane == 0) sdot[tt] = skq;
+    for (int u = 0; u < U; ++u) {
+      const int idx = threadIdx.x + 128 * u, tt = idx / VEC, c = (idx % VEC) * 8;
+      float4* dk4 = reinterpret_cast<float4*>(&sk[tt][c]);
+      float4* dq4 = reinterpret_cast<float4*>(&sq[tt][c]);
+      const T* k = raw[u].v;
+      const T* q = raw[U + u].v;
+      const float nk = len[u].x, nq = len[u].y;
+      dk4[0] = make_float4(act_f32(k[0]) * nk, act_f32(k[1]) * nk, act_f32(k[2]) * nk, act_f32(k[3]) * nk);
+      dk4[1] = make_float4(act_f32(k[4]) * nk, act_f32(k[5]) * nk, act_f32(k[6]) * nk, act_f32(k[7]) * nk);
+      dq4[0] = make_float4(act_f32(q[0]) * nq, act_f32(q[1]) * nq, act_f32(q[2]) * nq, act_f32(q[3]) * nq);
+      dq4[1] = make_float4(act_f32(q[4]) * nq, act_f32(q[5]) * nq, act_f32(q[6]) * nq, act_f32(q[7]) * nq);
     }
-    if (threadIdx.x < CH) { sgate[0][threadIdx.x] = ga; sgate[1][threadIdx.x] = gb; }
+#pragma unroll
+    for (int u = 0; u < CH * COLS / 128; ++u) {
+      const int idx = threadIdx.x + 128 * u;
+      sv[idx / COLS][idx % COLS] = act_f32(rv[u]);
+    }
+    if (threadIdx.x < NB * (GDN_COEF / 4)) reinterpret_cast<float4*>(&scoef[0][0])[threadIdx.x] = rc;
     __syncthreads();
     if (f0 + CH < t1) fetch(f0 + CH);
     const int n = min(CH, t1 - f0);
-    for (int tt = 0; tt < n; ++tt) {
-      const float decay = sgate[0][tt], bt = sgate[1][tt], kq = sdot[tt];
-      const float2 vj = *reinterpret_cast<const float2*>(&sv[tt][jj]);
-      const float4* k4 = reinterpret_cast<const float4*>(sk[tt]) + sp;
-      const float4* q4 = reinterpret_cast<const float4*>(sq[tt]) + sp;
-      float4 kk[G4];
-      float m0a = 0.f, m0b = 0.f, m1a = 0.f, m1b = 0.f, r0a = 0.f, r0b = 0.f, r1a = 0.f, r1b = 0.f;
+    for (int blk = 0; blk * BLK < n; ++blk) {
+      const int tt = blk * BLK;
+      float kk[BLK][NPT], val[16];
 #pragma unroll
-      for (int i = 0; i < G4; ++i) {
-        kk[i] = k4[i * 8];
-        const float4 qq = q4[i * 8];
-        m0a = fmaf(c0[4 * i], kk[i].x, m0a); m1a = fmaf(c1[4 * i], kk[i].x, m1a);
-        m0b = fmaf(c0[4 * i + 1], kk[i].y, m0b); m1b = fmaf(c1[4 * i + 1], kk[i].y, m1b);
-        m0a = fmaf(c0[4 * i + 2], kk[i].z, m0a); m1a = fmaf(c1[4 * i + 2], kk[i].z, m1a);
-        m0b = fmaf(c0[4 * i + 3], kk[i].w, m0b); m1b = fmaf(c1[4 * i + 3], kk[i].w, m1b);
-        r0a = fmaf(c0[4 * i], qq.x, r0a); r1a = fmaf(c1[4 * i], qq.x, r1a);
-        r0b = fmaf(c0[4 * i + 1], qq.y, r0b); r1b = fmaf(c1[4 * i + 1], qq.y, r1b);
-        r0a = fmaf(c0[4 * i + 2], qq.z, r0a); r1a = fmaf(c1[4 * i + 2], qq.z, r1a);
-        r0b = fmaf(c0[4 * i + 3], qq.w, r0b); r1b = fmaf(c1[4 * i + 3], qq.w, r1b);
-      }
-      float m0 = m0a + m0b, m1 = m1a + m1b, r0 = r0a + r0b, r1 = r1a + r1b;
+      for (int t = 0; t < BLK; ++t) {
+        const float4* k4 = reinterpret_cast<const float4*>(sk[tt + t]) + sp;
+        const float4* q4 = reinterpret_cast<const float4*>(sq[tt + t]) + sp;
+        float m0 = 0.f, m1 = 0.f, r0 = 0.f, r1 = 0.f;
 #pragma unroll
-      for (int o = 1; o < 8; o <<= 1) {
-        m0 += __shfl_xor_sync(0xffffffffu, m0, o);
-        m1 += __shfl_xor_sync(0xffffffffu, m1, o);
-        r0 += __shfl_xor_sync(0xffffffffu, r0, o);
-        r1 += __shfl_xor_sync(0xffffffffu, r1, o);
+        for (int i = 0; i < G4; ++i) {
+          const float4 kv = k4[i * 16], qv = q4[i * 16];
+          kk[t][4 * i] = kv.x; kk[t][4 * i + 1] = kv.y; kk[t][4 * i + 2] = kv.z; kk[t][4 * i + 3] = kv.w;
+          m0 = fmaf(c0[4 * i], kv.x, m0); m1 = fmaf(c1[4 * i], kv.x, m1); r0 = fmaf(c0[4 * i], qv.x, r0); r1 = fmaf(c1[4 * i], qv.x, r1);
+          m0 = fmaf(c0[4 * i + 1], kv.y, m0); m1 = fmaf(c1[4 * i + 1], kv.y, m1); r0 = fmaf(c0[4 * i + 1], qv.y, r0); r1 = fmaf(c1[4 * i + 1], qv.y, r1);
+          m0 = fmaf(c0[4 * i + 2], kv.z, m0); m1 = fmaf(c1[4 * i + 2], kv.z, m1); r0 = fmaf(c0[4 * i + 2], qv.z, r0); r1 = fmaf(c1[4 * i + 2], qv.z, r1);
+          m0 = fmaf(c0[4 * i + 3], kv.w, m0); m1 = fmaf(c1[4 * i + 3], kv.w, m1); r0 = fmaf(c0[4 * i + 3], qv.w, r0); r1 = fmaf(c1[4 * i + 3], qv.w, r1);
+        }
+        val[2 * t] = m0; val[2 * t + 1] = m1; val[8 + 2 * t] = r0; val[8 + 2 * t + 1] = r1;
       }
-      const float d0 = (vj.x - decay * m0) * bt, d1 = (vj.y - decay * m1) * bt;
 #pragma unroll
-      for (int i = 0; i < G4; ++i) {
-        c0[4 * i] = fmaf(kk[i].x, d0, decay * c0[4 * i]); c1[4 * i] = fmaf(kk[i].x, d1, decay * c1[4 * i]);
-        c0[4 * i + 1] = fmaf(kk[i].y, d0, decay * c0[4 * i + 1]); c1[4 * i + 1] = fmaf(kk[i].y, d1, decay * c1[4 * i + 1]);
-        c0[4 * i + 2] = fmaf(kk[i].z, d0, decay * c0[4 * i + 2]); c1[4 * i + 2] = fmaf(kk[i].z, d1, decay * c1[4 * i + 2]);
-        c0[4 * i + 3] = fmaf(kk[i].w, d0, decay * c0[4 * i + 3]); c1[4 * i + 3] = fmaf(kk[i].w, d1, decay * c1[4 * i + 3]);
+      for (int o = 8; o > 0; o >>= 1) {
+        const bool up = (sp & o) != 0;
+#pragma unroll
+        for (int i = 0; i < o; ++i) {
+          const float send = up ? val[i] : val[i + o], keep = up ? val[i + o] : val[i];
+          val[i] = keep + __shfl_xor_sync(0xffffffffu, send, o);
+        }
       }
-      if (sp == 0) {
-        T* dst = p.out + (size_t(f0 + tt) * Hv + h) * dv + j;
-        if (live0) dst[0] = act_from<T>(fmaf(decay, r0, kq * d0));
-        if (live1) dst[1] = act_from<T>(fmaf(decay, r1, kq * d1));
+      const float mine = val[0];                           // sum number sp: m_t of column c at 2 t + c, r_t at 8 + 2 t + c
+      const float* co = scoef[blk];
+      const float4 dec = *reinterpret_cast<const float4*>(co + 24), to_end = *reinterpret_cast<const float4*>(co + 28);
+      const float4 beta = *reinterpret_cast<const float4*>(co + 32), kk0 = *reinterpret_cast<const float4*>(co);
+      const float2 kk1 = *reinterpret_cast<const float2*>(co + 4);
+      float d[BLK][2];
+#pragma unroll
+      for (int c = 0; c < 2; ++c) {
+        const float v0 = sv[tt][jj + c], v1 = sv[tt + 1][jj + c], v2 = sv[tt + 2][jj + c], v3 = sv[tt + 3][jj + c];
+        const float m0 = __shfl_sync(0xffffffffu, mine, c, 16), m1 = __shfl_sync(0xffffffffu, mine, 2 + c, 16);
+        const float m2 = __shfl_sync(0xffffffffu, mine, 4 + c, 16), m3 = __shfl_sync(0xffffffffu, mine, 6 + c, 16);
+        d[0][c] = (v0 - dec.x * m0) * beta.x;
+        d[1][c] = (v1 - dec.y * m1 - kk0.x * d[0][c]) * beta.y;
+        d[2][c] = (v2 - dec.z * m2 - kk0.y * d[0][c] - kk0.z * d[1][c]) * beta.z;
+        d[3][c] = (v3 - dec.w * m3 - kk0.w * d[0][c] - kk1.x * d[1][c] - kk1.y * d[2][c]) * beta.w;
+      }
+      if (sp >= 8) {
+        const int t = (sp - 8) >> 1, c = sp & 1;
+        const float4 w = *reinterpret_cast<const float4*>(co + 8 + 4 * t);
+        float o = co[24 + t] * mine;
+        o = fmaf(w.x, c ? d[0][1] : d[0][0], o);
+        if (t > 0) o = fmaf(w.y, c ? d[1][1] : d[1][0], o);      // (a later token's values stay out, whatever they are)
+        if (t > 1) o = fmaf(w.z, c ? d[2][1] : d[2][0], o);
+        if (t > 2) o = fmaf(w.w, c ? d[3][1] : d[3][0], o);
+        if (tt + t < n && (c ? live1 : live0)) p.out[(size_t(f0 + tt + t) * Hv + h) * dv + j + c] = act_from<T>(o);
+      }
+      const float e[BLK] = {to_end.x, to_end.y, to_end.z, to_end.w};
+#pragma unroll
+      for (int i = 0; i < NPT; ++i) { c0[i] *= dec.w; c1[i] *= dec.w; }
+#pragma unroll
+      for (int t = 0; t < BLK; ++t) {
+        const float e0 = e[t] * d[t][0], e1 = e[t] * d[t][1];
+#pragma unroll
+        for (int i = 0; i < NPT; ++i) { c0[i] = fmaf(kk[t][i], e0, c0[i]); c1[i] = fmaf(kk[t][i], e1, c1[i]); }
       }
     }
   }
@@ -314,24 +441,35 @@ static bool LaunchGdnDecode(const GdnParams<T>& p, int B, int splits, cudaStream
                          : launch_pdl(gated_delta_kernel<T, NPT, false>, grid, block, 0, s, p);
 }
 template <typename T, int NPT, int CH>
-static bool LaunchGdnChunk(const GdnParams<T>& p, int B, cudaStream_t s) {
-  return launch_pdl(gated_delta_chunk_kernel<T, NPT, CH>, dim3(B, p.Hv, (p.dv + 31) / 32), dim3(128), 0, s, p);
+static bool LaunchGdnChunk(const GdnParams<T>& p, int B, int tokens, void* scratch, cudaStream_t s) {
+  float* coef = static_cast<float*>(scratch);
+  float2* lengths = reinterpret_cast<float2*>(coef + gdn_blocks(tokens, B) * p.Hv * GDN_COEF);
+  const int vec = p.dk % 8 == 0 && ((reinterpret_cast<uintptr_t>(p.q) | reinterpret_cast<uintptr_t>(p.k) | size_t(p.tok_stride_qk) * sizeof(T)) & 15) == 0;
+  return launch_pdl(gdn_prepare_kernel<T>, dim3(unsigned(gdn_blocks(tokens, B)), (p.Hv + 7) / 8), dim3(256), 0, s, p, B, lengths, coef) &&
+         launch_pdl(gated_delta_chunk_kernel<T, NPT, CH>, dim3(B, p.Hv, (p.dv + 15) / 16), dim3(128), 0, s, p, static_cast<const float2*>(lengths),
+                    static_cast<const float*>(coef), vec);
+}
+
+// Bytes of scratch that a launch of the chunk kernel over `tokens` tokens of `requests` requests needs (16-byte aligned).
+OGB_API long long ogb_gated_delta_scratch_bytes(int tokens, int requests, int Hk, int Hv) {
+  return (gdn_blocks(tokens, requests) * Hv * GDN_COEF + 2ll * tokens * Hk) * 4;
 }
 
 // max_q_len: the most tokens a request of the launch feeds (1: the decode kernel; 0: unknown, treated as a prompt)
+// scratch: ogb_gated_delta_scratch_bytes(tokens, B, Hk, Hv) bytes, or null: the decode kernel walks the tokens
 template <typename T>
-static int LaunchGatedDelta(const GdnParams<T>& p, int B, int max_q_len, void* stream) {
+static int LaunchGatedDelta(const GdnParams<T>& p, int B, int tokens, int max_q_len, void* scratch, void* stream) {
   if (B <= 0) return 0;
   const int dk = p.dk, dv = p.dv;
   if (p.Hk <= 0 || p.Hv % p.Hk || dv <= 0 || dk <= 0) return -1;
   if (dk > GDN_MAX_DK) return -5;
   auto s = static_cast<cudaStream_t>(stream);
   bool ok;
-  if (max_q_len != 1 && dk <= 256) {
-    if (dk <= 32) ok = LaunchGdnChunk<T, 4, 32>(p, B, s);
-    else if (dk <= 64) ok = LaunchGdnChunk<T, 8, 32>(p, B, s);
-    else if (dk <= 128) ok = LaunchGdnChunk<T, 16, 32>(p, B, s);
-    else ok = LaunchGdnChunk<T, 32, 16>(p, B, s);
+  if (max_q_len != 1 && dk <= 256 && scratch) {
+    if (reinterpret_cast<uintptr_t>(scratch) & 15) return -1;
+    if (dk <= 64) ok = LaunchGdnChunk<T, 4, 32>(p, B, tokens, scratch, s);
+    else if (dk <= 128) ok = LaunchGdnChunk<T, 8, 32>(p, B, tokens, scratch, s);
+    else ok = LaunchGdnChunk<T, 16, 16>(p, B, tokens, scratch, s);
     return ok ? 0 : -4;
   }
   // measured at Qwen3.5 shapes: 32 rows per thread 51 us, 16 rows 63 us, 64 rows 54 us (64 requests)
@@ -342,8 +480,8 @@ static int LaunchGatedDelta(const GdnParams<T>& p, int B, int max_q_len, void* s
 }
 
 OGB_API int ogb_gated_delta(const void* q, const void* k, const void* v, const float* g, const float* beta, float* state, const int32_t* slots,
-                            const int32_t* cu_seqlens, const int32_t* past_lens, void* out, int B, int Hk, int Hv, int dk, int dv, int max_q_len,
-                            void* stream) {
+                            const int32_t* cu_seqlens, const int32_t* past_lens, void* out, int B, int Hk, int Hv, int dk, int dv, int tokens,
+                            int max_q_len, void* scratch, void* stream) {
   using T = __nv_bfloat16;
   GdnParams<T> p{};
   p.q = static_cast<const T*>(q); p.k = static_cast<const T*>(k); p.v = static_cast<const T*>(v);
@@ -352,14 +490,14 @@ OGB_API int ogb_gated_delta(const void* q, const void* k, const void* v, const f
   p.state = state; p.slot_stride = static_cast<long long>(Hv) * dk * dv;
   p.slots = slots; p.cu_seqlens = cu_seqlens; p.past_lens = past_lens; p.out = static_cast<T*>(out);
   p.Hk = Hk; p.Hv = Hv; p.dv = dv; p.dk = dk;
-  return LaunchGatedDelta(p, B, max_q_len, stream);
+  return LaunchGatedDelta(p, B, tokens, max_q_len, scratch, stream);
 }
 
 template <typename T>
 static int GatedDeltaFused(const void* conv, long long conv_stride, long long q_off, long long k_off, long long v_off, const void* ba,
                            long long ba_stride, long long b_off, long long a_off, const float* neg_exp_a, const float* dt_bias, float q_scale,
                            float l2_eps, float* state, long long slot_stride, const int32_t* slots, const int32_t* cu_seqlens,
-                           const int32_t* past_lens, void* out, int B, int Hk, int Hv, int dk, int dv, int max_q_len, void* stream) {
+                           const int32_t* past_lens, void* out, int B, int Hk, int Hv, int dk, int dv, int tokens, int max_q_len, void* scratch, void* stream) {
   GdnParams<T> p{};
   auto c = static_cast<const T*>(conv);
   auto r = static_cast<const T*>(ba);
@@ -369,7 +507,7 @@ static int GatedDeltaFused(const void* conv, long long conv_stride, long long q_
   p.state = state; p.slot_stride = slot_stride > 0 ? slot_stride : static_cast<long long>(Hv) * dk * dv;
   p.slots = slots; p.cu_seqlens = cu_seqlens; p.past_lens = past_lens; p.out = static_cast<T*>(out);
   p.Hk = Hk; p.Hv = Hv; p.dv = dv; p.dk = dk;
-  return LaunchGatedDelta(p, B, max_q_len, stream);
+  return LaunchGatedDelta(p, B, tokens, max_q_len, scratch, stream);
 }
 
 // The recurrence fed straight from the layer's tensors: q / k / v are column ranges of the convolved projection `conv` [T, row
@@ -380,11 +518,11 @@ OGB_API int ogb_gated_delta_fused(const void* conv, long long conv_stride, long 
                                   long long ba_stride, long long b_off, long long a_off, const float* neg_exp_a, const float* dt_bias,
                                   float q_scale, float l2_eps, float* state, long long slot_stride, const int32_t* slots,
                                   const int32_t* cu_seqlens, const int32_t* past_lens, void* out, int B, int Hk, int Hv, int dk, int dv,
-                                  int max_q_len, int fp32, void* stream) {
+                                  int tokens, int max_q_len, int fp32, void* scratch, void* stream) {
   return fp32 ? GatedDeltaFused<float>(conv, conv_stride, q_off, k_off, v_off, ba, ba_stride, b_off, a_off, neg_exp_a, dt_bias, q_scale, l2_eps,
-                                       state, slot_stride, slots, cu_seqlens, past_lens, out, B, Hk, Hv, dk, dv, max_q_len, stream)
+                                       state, slot_stride, slots, cu_seqlens, past_lens, out, B, Hk, Hv, dk, dv, tokens, max_q_len, scratch, stream)
               : GatedDeltaFused<__nv_bfloat16>(conv, conv_stride, q_off, k_off, v_off, ba, ba_stride, b_off, a_off, neg_exp_a, dt_bias, q_scale,
-                                               l2_eps, state, slot_stride, slots, cu_seqlens, past_lens, out, B, Hk, Hv, dk, dv, max_q_len, stream);
+                                               l2_eps, state, slot_stride, slots, cu_seqlens, past_lens, out, B, Hk, Hv, dk, dv, tokens, max_q_len, scratch, stream);
 }
 
 OGB_API int ogb_gdn_gate_norm(const void* o, const void* z, long long z_stride, const float* w, float eps, void* out, long long out_stride, int T,

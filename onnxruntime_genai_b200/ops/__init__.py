@@ -582,6 +582,11 @@ def causal_conv(x, weight, bias, cache, slots, positions, cu_seqlens, past_lens,
     return out
 
 
+def _gated_delta_scratch(T, B, Hk, Hv, max_q_len, device):
+    """Scratch of the recurrence's prompt kernel (lengths and block coefficients); a decode step needs none."""
+    return None if max_q_len == 1 else torch.empty(_lib.lib().ogb_gated_delta_scratch_bytes(T, B, Hk, Hv), dtype=torch.uint8, device=device)
+
+
 def gated_delta(q, k, v, g, beta, state, slots, cu_seqlens, past_lens, max_q_len: int = 0):
     """Gated-delta-rule recurrence of a linear-attention layer over packed sequences (see ops/reference.py::gated_delta).
     state [slots, Hv, dk, dv] fp32 is updated in place.  max_q_len: most tokens of one request (1 selects the decode kernel, 0: not
@@ -595,14 +600,15 @@ def gated_delta(q, k, v, g, beta, state, slots, cu_seqlens, past_lens, max_q_len
     gf, bf = g.float().contiguous(), beta.float().contiguous()
     out = torch.empty(T, Hv, dv, dtype=torch.bfloat16, device=q.device)
     B = past_lens.shape[0]
+    scratch = _gated_delta_scratch(T, B, Hk, Hv, max_q_len, q.device)
     _lib.check(_lib.lib().ogb_gated_delta(_ptr(q), _ptr(k), _ptr(v), _ptr(gf), _ptr(bf), _ptr(state), _ptr(slots), _ptr(cu_seqlens), _ptr(past_lens),
-                                          _ptr(out), B, Hk, Hv, dk, dv, int(max_q_len), _stream()), "gated_delta")
+                                          _ptr(out), B, Hk, Hv, dk, dv, T, int(max_q_len), _ptr(scratch), _stream()), "gated_delta")
     return out
 
 
 def gated_delta_layer(conv, proj, cd, vd, Hk, Hv, dk, dv, neg_exp_a, dt_bias, norm_w, norm_eps, state, slots, cu_seqlens, past_lens,
                       max_q_len: int = 0, l2_eps: float = 0.0, out=None):
-    """The part of a gated-delta-net layer between its convolution and its output projection, as two kernels on CUDA tensors (bf16 or
+    """The part of a gated-delta-net layer between its convolution and its output projection, as two (prompts: three) kernels on CUDA tensors (bf16 or
     fp32): conv [T, cd] = silu(conv1d([q | k | v])), proj [T, cd + vd + 2 Hv] = the input projection [qkv | z | b | a].  q and k are
     L2-normalised per head (q also scaled by dk^-0.5), beta = sigmoid(b), log-decay = neg_exp_a * softplus(a + dt_bias), the
     recurrence updates `state` in place, and the result is RMS-normalised per value head, weighted and gated by silu(z).
@@ -614,10 +620,11 @@ def gated_delta_layer(conv, proj, cd, vd, Hk, Hv, dk, dv, neg_exp_a, dt_bias, no
     kd, f32 = Hk * dk, int(conv.dtype == torch.float32)
     o = torch.empty(T, Hv, dv, dtype=conv.dtype, device=conv.device)
     B = past_lens.shape[0]
+    scratch = _gated_delta_scratch(T, B, Hk, Hv, max_q_len, conv.device)
     _lib.check(_lib.lib().ogb_gated_delta_fused(_ptr(conv), conv.stride(0), 0, kd, 2 * kd, _ptr(proj), proj.stride(0), cd + vd, cd + vd + Hv,
                                                 _ptr(neg_exp_a), _ptr(dt_bias), float(dk) ** -0.5, float(l2_eps), _ptr(state), state.stride(0),
-                                                _ptr(slots), _ptr(cu_seqlens), _ptr(past_lens), _ptr(o), B, Hk, Hv, dk, dv, int(max_q_len), f32,
-                                                _stream()), "gated_delta_fused")
+                                                _ptr(slots), _ptr(cu_seqlens), _ptr(past_lens), _ptr(o), B, Hk, Hv, dk, dv, T, int(max_q_len), f32,
+                                                _ptr(scratch), _stream()), "gated_delta_fused")
     if out is None:
         out = torch.empty(T, Hv * dv, dtype=conv.dtype, device=conv.device)
     z = proj[:, cd:cd + vd]
