@@ -34,8 +34,8 @@
 // have to be consumed every 190 cycles to keep up with HBM.  More expander warps, more expanded tiles in flight, a deeper
 // activation ring, tensor-map loads and four independent accumulators each left the time within 8 %.  The kernel
 // therefore streams its weights at about 0.33 of the HBM rate (1.25x faster than the bf16 experts, which move 3.8x the
-// bytes at the full rate).  It serves the larger token tiles (prompts); the 16-token tiles of decode steps go to the
-// streaming kernel further down, which keeps the expanded weights in registers.
+// bytes at the full rate).  Tiles of 32 tokens and more (prompts) run on pairs of SMs (gemm_pair.cu), the 16-token tiles of decode steps of the fp16
+// form on the streaming kernel further down, which keeps the expanded weights in registers: this kernel serves the 16-token tiles of the bf16 form.
 #include <cstdlib>
 
 #include "gemm_common.cuh"
@@ -524,12 +524,11 @@ static int LaunchFp4V(const CUtensorMap& ta, const CUtensorMap& tw, int w_by_tma
 template <int BT, bool HALF>
 static int LaunchFp4(const CUtensorMap& ta, const CUtensorMap& tw, int w_by_tma, const uint8_t* wp, int n_tiles, int skip, const GemmParams& p,
                      dim3 grid, cudaStream_t stream) {
-  // 16-token tiles: four expanded tiles in flight, the expander warps in two groups that alternate k-blocks, four
-  // accumulators; larger tiles: two expanded tiles, one group, one accumulator.  Measured on B200 (gate/up of gpt-oss-20b,
-  // 32 tokens): 131 us against 142 us for the single-group forms - the kernel is bound by the rate at which the tensor
-  // core retires 128 x 16 x 16 instructions, not by the expansion, the copies or the accumulator chain.
-  if constexpr (BT <= 16) return LaunchFp4V<BT, HALF, 4, 2, 4>(ta, tw, w_by_tma, wp, n_tiles, skip, p, grid, stream);
-  return LaunchFp4V<BT, HALF, 2, 1, 1>(ta, tw, w_by_tma, wp, n_tiles, skip, p, grid, stream);
+  // Four expanded tiles in flight, the expander warps in two groups that alternate k-blocks, four accumulators.  Measured on B200 (gate/up of
+  // gpt-oss-20b, 32 tokens): 131 us against 142 us for the single-group forms - the kernel is bound by the rate at which the issuing warp
+  // passes over stages, not by the expansion, the copies or the accumulator chain.
+  static_assert(BT == 16, "larger token tiles run in gemm_pair.cu");
+  return LaunchFp4V<BT, HALF, 4, 2, 4>(ta, tw, w_by_tma, wp, n_tiles, skip, p, grid, stream);
 }
 
 }  // namespace ogb

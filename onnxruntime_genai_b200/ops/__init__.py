@@ -405,7 +405,7 @@ def linear(x, w, bias=None, residual=None, out_fp32=False, out=None, splits=0, a
     fused = None
     if norm_eps > 0:
         if x.shape[0] > FUSED_MAX_TOKENS:
-            x = rms_scale(x, norm_eps)     # prefill-sized steps run the persistent kernel: normalise first
+            x = rms_scale(x, norm_eps)     # prompt-sized steps run the paired kernel: normalise first
         else:
             fused = _lib.GemmFused(norm_eps=float(norm_eps))
     rows_out = x.shape[0]

@@ -104,7 +104,7 @@ class TensorParallel:
     def fused_ok(self, x: torch.Tensor, n_out: Optional[int] = None) -> bool:
         """True when the GEMM + all-reduce kernel can take this activation: decode-sized token counts with the flagged-line
         protocol; with NVLS switched on and OGB_TP_FUSED_PREFILL=1 also any step whose [tokens, n_out] output fits the
-        multicast plane (measured slower than the persistent GEMM followed by a stand-alone all-reduce at two ranks)."""
+        multicast plane (measured slower than a persistent GEMM followed by a stand-alone all-reduce at two ranks)."""
         if self.comm is None or not x.is_cuda:
             return False
         if x.shape[0] <= self.comm.max_tokens:
