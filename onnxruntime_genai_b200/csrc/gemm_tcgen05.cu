@@ -4,7 +4,7 @@
 // The weight is the UMMA "M" operand (128 output features per CTA) and the activations are the
 // UMMA "N" operand (16..256 tokens), so the same kernel serves decode (few tokens, bandwidth bound:
 // every SM streams weight tiles through a deep TMA pipeline, two CTAs per SM) and prefill
-// (256-token tiles, compute bound).  Both operands are K-major in shared memory with the 128-byte
+// (256-token tiles of products that gemm_pair.cu leaves here).  Both operands are K-major in shared memory with the 128-byte
 // swizzle written by TMA; accumulators live in tensor memory and are read back with tcgen05.ld.
 //
 // Warp roles (192 threads): warp 0 = TMA producer, warp 1 = MMA issuer, both as whole warps with one elected lane,
@@ -423,7 +423,7 @@ const CommParams* ogb_comm_params(int device) { return (device >= 0 && device < 
 
 OGB_API int ogb_gemm_token_tile(int M, int dual) {
   (void)dual;
-  // prefill-sized problems: 256-token tiles, one CTA per SM
+  // more than 128 tokens: 256-token tiles, one CTA per SM
   if (M <= 16) return 16;
   if (M <= 32) return 32;
   if (M <= 64) return 64;
