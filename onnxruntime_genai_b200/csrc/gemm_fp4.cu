@@ -564,7 +564,10 @@ OGB_API int ogb_moe_gemm_fp4(const void* A, int lda, const void* Wpacked, void* 
   if (act_pair && (N % 128)) return -1;
   if (max_tiles > 65535) return -1;
   static const int pdl_enabled = [] { const char* e = getenv("OGB_PDL"); return (e && e[0] == '0') ? 0 : 1; }();
+  // Refused here, before anything is launched: neither the tensor maps nor the paired kernel would notice (its instruction takes tokens in steps of 32,
+  // a CTA holds half of them in groups of eight).
   const int bt = token_tile;
+  if (bt != 16 && bt != 32 && bt != 64 && bt != 128 && bt != 256) return -5;
   CUtensorMap ta = {};
   if (!row_map && !MakeMapBf16(&ta, A, rows_total, K, lda, bt)) return -2;
   GemmParams p = {};
