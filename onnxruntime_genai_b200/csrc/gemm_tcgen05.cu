@@ -456,7 +456,9 @@ OGB_API int ogb_gemm_auto_splits(int M, int N, int K, int dual, int sm_count) {
     const int kbs = total_kb / s;
     // 8 partitions: long k ranges whose 4-way split would not fit one CTA per SM (that form runs the deep pipeline: down
     // 25.1 us at s=4 against 27.7 at s=8), or launches so small that even 8 partitions leave one CTA per SM
-    if (s == 8 && bt == 256) break;       // (eight CTAs of a cluster at one per SM: a second wave, N 2048, K 8192 40 us against 26 with four)
+    // 256-token tiles hold one CTA per SM: 14 clusters of eight are resident at once, 16 are not (us, eight / four: M 200, N 512, K 14336 21.7 / 30.6,
+    // N 896, K 4864 15.7 / 18.7; N 2048, K 8192 40 / 26)
+    if (s == 8 && bt == 256 && tiles > 14) break;
     const bool ok = s <= 4 ? kbs >= 2 : ((kbs >= 16 && tiles * 4 > sm_count) || (tiles * s <= sm_count && kbs >= 8));
     if (ok) best = s;
   }
