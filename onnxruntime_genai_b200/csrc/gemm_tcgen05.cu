@@ -647,9 +647,10 @@ OGB_API int ogb_gemm_bf16_fused(const void* A, int lda, const void* W, int ldw, 
   }
   // Prompt-sized products run on pairs of SMs.  The (tiles x k-splits) form below keeps those whose few tiles leave pairs idle over a long k range; its
   // CTAs take about 420 ns per k-block (128-token tiles: 470, two CTAs per SM) and 10 us beside.  Weights from HBM, us, pairs / splits: M 233, N 4096, K 4096
-  // 19 / 21, K 14336 56 / 39; M 80, N 4096, K 14336 54 / 35; M 80, N 16384, K 2048 16 / 23; M 200, N 4096, K 960 8 / 15.  Short k ranges stay here although
-  // pairs are faster (K 512 5 / 13): the gathered form of a product, which only this kernel has, gives the same bits as the plain one.
-  if (!extras && !p.comm_epilogue && p.ag_rows == 0 && (pair_tiles > 0 || (auto_split && M > 64 && (M > 256 || total_kb > 8)))) {
+  // 19 / 21, K 14336 56 / 39; M 80, N 4096, K 14336 54 / 35; M 80, N 16384, K 2048 16 / 23; M 200, N 384, K 512 3.8 / 12.9; M 128, N 4096, K 512 5.5 / 11.5;
+  // M 256, N 14336, K 64 8.3 / 24.4.  The paired form sums k in one accumulator, the other one per split: the gathered form of a product, which only this
+  // kernel has, repeats the bits of the plain one at the same number of splits.
+  if (!extras && !p.comm_epilogue && p.ag_rows == 0 && (pair_tiles > 0 || (auto_split && M > 64))) {
     const double slots = bt == 128 ? 2.0 * sm_count : 1.0 * sm_count, ctas = double(n_tiles) * m_tiles * splits;
     const double waves = double((long long)((ctas + slots - 1) / slots));
     if (pair_tiles > 0 || PairBf16Ns(M, N, total_kb) < waves * kb_per * (bt == 128 ? 470.0 : 420.0) + 10000.0)

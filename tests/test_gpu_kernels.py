@@ -127,19 +127,24 @@ def test_standalone_collectives_world_of_one():
 @pytest.mark.parametrize("M,N,K,pair", [(64, 512, 1024, False), (5, 256, 4096, False), (200, 384, 512, False), (48, 512, 256, True)])
 def test_gemm_all_gather_fused_world_of_one(M, N, K, pair):
     """all-gather -> GEMM: activations pushed as flagged lines, tiles assembled inside the GEMM (swizzled layout,
-    row / k tails, split-K clusters), against the plain GEMM on the same data."""
+    row / k tails, split-K clusters), against the plain GEMM on the same data: bit for bit at the gathered form's number of splits (which is
+    the plain one's own choice up to 64 tokens; larger ones may run on pairs of SMs and sum in another order)."""
     from onnxruntime_genai_b200.parallel.symm import LocalComm
     comm = LocalComm(torch.device("cuda", 0))
     try:
         x, w = _rand(M, K, seed=71), _rand(N, K, std=0.05, seed=72)
         if pair:
             w = ops.interleave_gate_up(w)
+        splits = 0 if M <= 64 else ops._lib.lib().ogb_gemm_auto_splits(M, N, K, 0, ops.workspace(x.device).sm_count)
         for _ in range(3):
             comm.all_gather_push(x)
             y = ops.linear_gathered(M, w, act_pair=pair)
-            want = ops.gate_up_act(x, w, interleaved=True) if pair else ops.linear(x, w)
+            want = ops.gate_up_act(x, w, interleaved=True, splits=splits) if pair else ops.linear(x, w, splits=splits)
             ops.check_kernel_status()
             assert torch.equal(y, want), f"max diff {(y.float() - want.float()).abs().max().item()}"
+            if not pair:      # the plain form of its own choice: 32-bit sums of K products in any order, half a place of bf16 on each side
+                bound = K * 2.0 ** -23 * (x.double().abs() @ w.double().abs().t()) + 2.0 ** -7 * want.double().abs()
+                assert ((ops.linear(x, w).double() - want.double()).abs() <= bound).all()
             assert torch.equal(comm.all_reduce(x), x)     # a waiting call between two pushes
     finally:
         comm.close()
