@@ -24,7 +24,7 @@
 // multiplier byte is scale code + 6 (the kernels subtract 118 to reach the fp16 exponent field of 2^(scale - 127)).
 //
 // Pipeline and epilogue are those of the int4 kernel (gemm_w4.cu): warp 0 streams records through a deep ring and the
-// activation tiles through a ring of their own (4 or 8 deep), warps 2..9 expand a record into the swizzled K-major tile,
+// activation tiles through a ring of their own, warps 2..9 expand a record into the swizzled K-major tile,
 // warp 1 issues tcgen05.mma into tensor memory, warps 2..5 run the epilogue; two CTAs per SM.  The tile list of
 // ogb_moe_sort selects the expert, first row and row count of each token tile.  Every wait is bounded.
 //
@@ -35,7 +35,8 @@
 // activation ring, tensor-map loads and four independent accumulators each left the time within 8 %.  The kernel
 // therefore streams its weights at about 0.33 of the HBM rate (1.25x faster than the bf16 experts, which move 3.8x the
 // bytes at the full rate).  Tiles of 32 tokens and more (prompts) run on pairs of SMs (gemm_pair.cu), the 16-token tiles of decode steps of the fp16
-// form on the streaming kernel further down, which keeps the expanded weights in registers: this kernel serves the 16-token tiles of the bf16 form.
+// form on the streaming kernel further down, which keeps the expanded weights in registers: this kernel serves the 16-token tiles of the bf16 form,
+// and of the fp16 form those whose K is above what the streaming kernel stages.
 #include <cstdlib>
 
 #include "gemm_common.cuh"
@@ -45,42 +46,40 @@
 namespace ogb {
 
 constexpr int FP4_THREADS = 320;   // warp 0 producer, warp 1 MMA issuer, warps 2..9 expanders (2..5 also run the epilogue)
-constexpr int FP4_DEQ_WARPS = 8;
+constexpr int FP4_BT = 16;         // tokens of a tile
+// Four expanded tiles in flight, the expander warps in two groups that alternate k-blocks (2..5 the even ones, 6..9 the odd ones, one thread per row),
+// four accumulators.  Measured on B200 (gate/up of gpt-oss-20b, 32 tokens): 131 us against 142 us for the single-group forms - the kernel is bound by
+// the rate at which the issuing warp passes over stages, not by the expansion, the copies or the accumulator chain.
+constexpr int FP4_WBUF = 4, FP4_GROUPS = 2;
+// Accumulators: consecutive tcgen05.mma into one accumulator run as a dependent chain (a 128 x 16 x 16 step is
+// latency, not work), so the four k-steps of a k-block go to four accumulators of FP4_BT columns, summed in the epilogue.
+constexpr int FP4_NACC = 4;
 
-template <int BT, int FP4_WBUF>
 struct Fp4Cfg {
-  static constexpr int A_TILE_BYTES = BT * GEMM_BLOCK_K * 2;
-  static constexpr bool TWO_PER_SM = BT <= 64;
-  static constexpr int BUDGET = TWO_PER_SM ? 100 * 1024 : 196 * 1024;
+  static constexpr int A_TILE_BYTES = FP4_BT * GEMM_BLOCK_K * 2;
+  static constexpr int BUDGET = 100 * 1024;      // two CTAs per SM
   // Activation tiles have their own, deeper ring: a tile is requested when the MMA that read the slot has finished, and
   // the copy takes most of a microsecond to arrive, so with two slots every k-block waited half that latency (the
   // kernel then ran at 0.3 of the HBM rate whatever the expansion cost).
-  static constexpr int A_STAGES = BT <= 32 ? 8 : 4;
+  static constexpr int A_STAGES = 8;
   static constexpr int FIXED = FP4_WBUF * W_TILE_BYTES + A_STAGES * A_TILE_BYTES;
-  static constexpr int MAX_RAW = (BUDGET - FIXED) / FP4_RECORD_BYTES;
   // a multiple of 4 records keeps the tiles behind the ring 1 KiB aligned (4 * 4352 = 17 KiB)
-  static constexpr int RAW = (MAX_RAW > 16 ? 16 : MAX_RAW) / 4 * 4;
-  // Accumulators: consecutive tcgen05.mma into one accumulator run as a dependent chain (a 128 x 16 x 16 step is
-  // latency, not work), so the four k-steps of a k-block go to NACC accumulators BT columns apart, summed in the epilogue.
-  static constexpr int NACC_MAX = BT <= 32 ? 4 : (BT <= 128 ? 2 : 1);
-  static constexpr int TMEM_COLS = (BT * NACC_MAX) < 32 ? 32 : BT * NACC_MAX;
+  static constexpr int RAW = (BUDGET - FIXED) / FP4_RECORD_BYTES / 4 * 4;
+  static constexpr int TMEM_COLS = FP4_BT * FP4_NACC;
   static constexpr int DATA_BYTES = RAW * FP4_RECORD_BYTES + FIXED;
   static constexpr int SMEM_BYTES = DATA_BYTES + 1024 + 512;
   static_assert(RAW >= 4, "raw ring too shallow");
   static_assert((RAW * FP4_RECORD_BYTES) % 1024 == 0, "swizzled tiles need 1 KiB alignment");
-  static_assert(BT * GEMM_BLOCK_N * 4 <= DATA_BYTES, "the parked fp32 tile must fit in the pipeline memory");
+  static_assert(FP4_BT * GEMM_BLOCK_N * 4 <= DATA_BYTES, "the parked fp32 tile must fit in the pipeline memory");
 };
 
-// FP4_WBUF: expanded weight tiles in flight; GROUPS: 1 = all eight expander warps share every k-block (two threads per
-// row), 2 = warps 2..5 take the even k-blocks and warps 6..9 the odd ones (one thread per row).
-template <int BT, bool HALF, int FP4_WBUF, int GROUPS, int NACC>
-__global__ void __launch_bounds__(FP4_THREADS, Fp4Cfg<BT, FP4_WBUF>::TWO_PER_SM ? 2 : 1)
-gemm_fp4_grouped_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_w,
-                        const uint8_t* __restrict__ wpacked, int n_tiles_per_expert, int w_by_tma, int skip_rows_le,
-                        const GemmParams p) {
-  using Cfg = Fp4Cfg<BT, FP4_WBUF>;
-  constexpr int RAW = Cfg::RAW;
-  constexpr int ARRIVALS = FP4_DEQ_WARPS / GROUPS;
+// HALF: fp16 activations and records in the fp16 layout
+template <bool HALF>
+__global__ void __launch_bounds__(FP4_THREADS, 2)
+gemm_fp4_grouped_kernel(const __grid_constant__ CUtensorMap tmap_a, const uint8_t* __restrict__ wpacked, int n_tiles_per_expert, const GemmParams p) {
+  using Cfg = Fp4Cfg;
+  constexpr int BT = FP4_BT, RAW = Cfg::RAW;
+  constexpr int ARRIVALS = 8 / FP4_GROUPS;       // expander warps of a k-block
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   uint8_t* raw_ring = smem;
@@ -107,7 +106,6 @@ gemm_fp4_grouped_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid
   const int row0 = p.grp.tile_row0[m_tile];
   const int rows = p.grp.tile_rows[m_tile];
   const int expert = p.grp.tile_expert[m_tile];
-  if (rows <= skip_rows_le) return;         // this tile belongs to the streaming kernel below (uniform over the CTA)
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < RAW; ++s) { mbar_init(&raw_full[s], 1); mbar_init(&raw_empty[s], ARRIVALS); }
@@ -117,7 +115,6 @@ gemm_fp4_grouped_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid
     *abort_flag = 0;
     mbar_fence_init();
     tma_prefetch_desc(&tmap_a);
-    tma_prefetch_desc(&tmap_w);
   }
   if (warp == 2) {
     tmem_alloc(tmem_slot, Cfg::TMEM_COLS);
@@ -135,13 +132,10 @@ gemm_fp4_grouped_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid
       // ------------------------------------------------------------ producer: packed records + activation tiles
       const uint8_t* rec0 = wpacked + (size_t(expert) * num_kb * n_tiles_per_expert + n_tile) * FP4_RECORD_BYTES;
       const size_t rec_stride = size_t(n_tiles_per_expert) * FP4_RECORD_BYTES;
-      // A record is 34 rows of 128 bytes: one untiled bulk copy, or (OGB_FP4_TMA=1) one box of a byte tensor map
-      const int rec_first = (expert * num_kb) * n_tiles_per_expert + n_tile;
       auto load_raw = [&](int i) {
         const int s = i % RAW;
         mbar_expect_tx(&raw_full[s], FP4_RECORD_BYTES);
-        if (w_by_tma) tma_load_2d(raw_ring + s * FP4_RECORD_BYTES, &tmap_w, &raw_full[s], 0, (rec_first + i * n_tiles_per_expert) * (FP4_RECORD_BYTES / 128));
-        else bulk_copy_g2s(raw_ring + s * FP4_RECORD_BYTES, rec0 + size_t(i) * rec_stride, FP4_RECORD_BYTES, &raw_full[s]);
+        bulk_copy_g2s(raw_ring + s * FP4_RECORD_BYTES, rec0 + size_t(i) * rec_stride, FP4_RECORD_BYTES, &raw_full[s]);
       };
       auto load_a = [&](int i) {
         const int s = i % A_ST;
@@ -180,52 +174,37 @@ gemm_fp4_grouped_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid
         const uint32_t w = smem_u32(w_ring + s * W_TILE_BYTES), a = smem_u32(a_ring + as * Cfg::A_TILE_BYTES);
 #pragma unroll
         for (int k = 0; k < GEMM_BLOCK_K / GEMM_UMMA_K; ++k)
-          umma_f16(tmem_base + uint32_t((k % NACC) * BT), umma_desc_sw128(w + k * GEMM_UMMA_K * 2), umma_desc_sw128(a + k * GEMM_UMMA_K * 2),
-                   idesc, (i > 0 || k >= NACC) ? 1u : 0u);
+          umma_f16(tmem_base + uint32_t((k % FP4_NACC) * BT), umma_desc_sw128(w + k * GEMM_UMMA_K * 2), umma_desc_sw128(a + k * GEMM_UMMA_K * 2),
+                   idesc, (i > 0 || k >= FP4_NACC) ? 1u : 0u);
         umma_commit(&w_empty[s]);
         umma_commit(&a_empty[as]);
       }
       if (ok) umma_commit(accum_bar);
     }
   } else {
-    // -------------------------------------------------------------- expanders: two threads per weight row of the tile,
-    // one block of 32 weights (16 bytes of nibbles, one multiplier byte) each; one arrival per warp on the barriers
+    // -------------------------------------------------------------- expanders: a thread per weight row of the tile; one arrival per warp on the barriers
     const int dt = threadIdx.x - 64;
     const int row = dt & 127;
-    constexpr int WORDS = 4 * GROUPS;                       // 32-bit words of nibbles per thread and k-block
-    const int group = GROUPS == 2 ? dt >> 7 : 0;            // which k-blocks this thread expands
-    const int part = GROUPS == 2 ? 0 : dt >> 7;             // which block of 32 of the row's 64 weights (GROUPS == 1)
-    for (int i = group; i < num_kb; i += GROUPS) {
+    for (int i = dt >> 7; i < num_kb; i += FP4_GROUPS) {
       const int rs = i % RAW, ws = i % FP4_WBUF;
       bool ok = mbar_wait_bounded(&raw_full[rs], (i / RAW) & 1, abort_flag);
       if (ok && i >= FP4_WBUF) ok = mbar_wait_bounded(&w_empty[ws], ((i / FP4_WBUF) & 1) ^ 1, abort_flag);
       if (!__all_sync(0xffffffffu, ok)) { fail(OGB_ERR_WAIT_TMA); break; }   // the warp gives up as one (it meets at __syncwarp below)
       const uint8_t* rec = raw_ring + rs * FP4_RECORD_BYTES;
-      uint32_t words[WORDS];
-#pragma unroll
-      for (int h = 0; h < WORDS / 4; ++h) {
-        const uint4 q = *reinterpret_cast<const uint4*>(rec + row * 32 + (part + h) * 16);
-        words[4 * h] = q.x; words[4 * h + 1] = q.y; words[4 * h + 2] = q.z; words[4 * h + 3] = q.w;
-      }
+      const uint4 q0 = *reinterpret_cast<const uint4*>(rec + row * 32), q1 = *reinterpret_cast<const uint4*>(rec + row * 32 + 16);
+      const uint32_t words[8] = {q0.x, q0.y, q0.z, q0.w, q1.x, q1.y, q1.z, q1.w};
       const uint32_t mul = *reinterpret_cast<const uint16_t*>(rec + GEMM_BLOCK_N * 32 + row * 2);   // exponent fields of the two multipliers
       uint8_t* dst = w_ring + ws * W_TILE_BYTES + row * 128;
       if constexpr (HALF) {
+        // word (q, b) of the record expands to the 16-byte chunk 4 b + q; the stored byte is code + 6, the fp16 field of 2^(code - 127) is code - 112
+        const uint32_t s0 = ((mul & 0xFFu) - 118u) * 0x04000400u, s1 = ((mul >> 8) - 118u) * 0x04000400u;
 #pragma unroll
-        for (int jj = 0; jj < WORDS; ++jj) {
-          const int rw = part * 4 + jj;                       // word of the record: (q, b) = (rw / 2, rw % 2)
-          const int j = 4 * (rw & 1) + (rw >> 1);             // the 16-byte chunk (8 k values) of the tile row it expands to
-          // the stored byte is code + 6; the fp16 exponent field of 2^(code - 127) is code - 112
-          const uint32_t m8 = ((rw & 1) ? (mul >> 8) : (mul & 0xFFu)) - 118u;
-          const uint32_t sb = (m8 << 10) | (m8 << 26);
-          *reinterpret_cast<uint4*>(dst + ((j ^ (row & 7)) << 4)) = deq_fp4_word_f16(words[jj], sb);
-        }
+        for (int q = 0; q < 8; ++q)
+          *reinterpret_cast<uint4*>(dst + (((4 * (q & 1) + (q >> 1)) ^ (row & 7)) << 4)) = deq_fp4_word_f16(words[q], (q & 1) ? s1 : s0);
       } else {
 #pragma unroll
-        for (int jj = 0; jj < WORDS; ++jj) {
-          const int j = part * 4 + jj;
-          const uint32_t m8 = j < 4 ? (mul & 0xFFu) : (mul >> 8);
-          *reinterpret_cast<uint4*>(dst + ((j ^ (row & 7)) << 4)) = deq_fp4_word_bf16(words[jj], m8);
-        }
+        for (int q = 0; q < 8; ++q)
+          *reinterpret_cast<uint4*>(dst + ((q ^ (row & 7)) << 4)) = deq_fp4_word_bf16(words[q], q < 4 ? (mul & 0xFFu) : (mul >> 8));
       }
       fence_proxy_async_smem();   // generic-proxy stores -> visible to the tensor core
       __syncwarp();
@@ -236,7 +215,7 @@ gemm_fp4_grouped_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid
     }
   }
 
-  gemm_epilogue<BT, 0>(p, smem, tmem_base, accum_bar, abort_flag, use_slot, n_tile, m_tile, row0, rows, expert * p.N, nullptr, NACC);
+  gemm_epilogue<BT, 0>(p, smem, tmem_base, accum_bar, abort_flag, use_slot, n_tile, m_tile, row0, rows, expert * p.N, nullptr, FP4_NACC);
 
   tc_fence_before();
   __syncthreads();
@@ -494,41 +473,13 @@ static int LaunchFp4Stream(const void* A, int lda, const int* row_map, const uin
 
 bool MakeMapBf16(CUtensorMap* out, const void* ptr, int rows, int cols, int ld, int box_rows);  // gemm_tcgen05.cu
 int LaunchPairFp4(const void* A, int lda, const uint8_t* packed, const GemmParams& p, int token_tile, int max_tiles, bool half, cudaStream_t stream);  // gemm_pair.cu
-bool MakeMapBytes128(CUtensorMap* out, const void* ptr, long long rows, int box_rows);          // gemm_tcgen05.cu
 
-template <int BT, bool HALF, int WBUF, int GROUPS, int NACC>
-static int LaunchFp4V(const CUtensorMap& ta, const CUtensorMap& tw, int w_by_tma, const uint8_t* wp, int n_tiles, int skip, const GemmParams& p,
-                      dim3 grid, cudaStream_t stream) {
-  using Cfg = Fp4Cfg<BT, WBUF>;
-  static_assert(NACC <= Fp4Cfg<BT, WBUF>::NACC_MAX, "not enough tensor memory for the accumulators");
-  auto kern = gemm_fp4_grouped_kernel<BT, HALF, WBUF, GROUPS, NACC>;
+template <bool HALF>
+static int LaunchFp4(const CUtensorMap& ta, const uint8_t* wp, int n_tiles, const GemmParams& p, dim3 grid, cudaStream_t stream) {
+  auto kern = gemm_fp4_grouped_kernel<HALF>;
   static bool configured[OGB_MAX_DEVICES] = {};
-  if (!set_max_dyn_smem(kern, Cfg::SMEM_BYTES, configured)) return -3;
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = grid;
-  cfg.blockDim = dim3(FP4_THREADS);
-  cfg.dynamicSmemBytes = Cfg::SMEM_BYTES;
-  cfg.stream = stream;
-  cudaLaunchAttribute attrs[1];
-  int na = 0;
-  if (p.pdl) {
-    attrs[na].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attrs[na].val.programmaticStreamSerializationAllowed = 1;
-    ++na;
-  }
-  cfg.attrs = attrs;
-  cfg.numAttrs = unsigned(na);
-  return cudaLaunchKernelEx(&cfg, kern, ta, tw, wp, n_tiles, w_by_tma, skip, p) == cudaSuccess ? 0 : -4;
-}
-
-template <int BT, bool HALF>
-static int LaunchFp4(const CUtensorMap& ta, const CUtensorMap& tw, int w_by_tma, const uint8_t* wp, int n_tiles, int skip, const GemmParams& p,
-                     dim3 grid, cudaStream_t stream) {
-  // Four expanded tiles in flight, the expander warps in two groups that alternate k-blocks, four accumulators.  Measured on B200 (gate/up of
-  // gpt-oss-20b, 32 tokens): 131 us against 142 us for the single-group forms - the kernel is bound by the rate at which the issuing warp
-  // passes over stages, not by the expansion, the copies or the accumulator chain.
-  static_assert(BT == 16, "larger token tiles run in gemm_pair.cu");
-  return LaunchFp4V<BT, HALF, 4, 2, 4>(ta, tw, w_by_tma, wp, n_tiles, skip, p, grid, stream);
+  if (!set_max_dyn_smem(kern, Fp4Cfg::SMEM_BYTES, configured)) return -3;
+  return launch_pdl(kern, grid, dim3(FP4_THREADS), Fp4Cfg::SMEM_BYTES, stream, ta, wp, n_tiles, p) ? 0 : -4;
 }
 
 }  // namespace ogb
@@ -568,8 +519,6 @@ OGB_API int ogb_moe_gemm_fp4(const void* A, int lda, const void* Wpacked, void* 
   // a CTA holds half of them in groups of eight).
   const int bt = token_tile;
   if (bt != 16 && bt != 32 && bt != 64 && bt != 128 && bt != 256) return -5;
-  CUtensorMap ta = {};
-  if (!row_map && !MakeMapBf16(&ta, A, rows_total, K, lda, bt)) return -2;
   GemmParams p = {};
   p.M = rows_total; p.N = N; p.K = K;
   p.total_kb = K / GEMM_BLOCK_K;
@@ -582,21 +531,19 @@ OGB_API int ogb_moe_gemm_fp4(const void* A, int lda, const void* Wpacked, void* 
   p.pdl = pdl_enabled;
   p.grp.tile_expert = tile_expert; p.grp.tile_row0 = tile_row0; p.grp.tile_rows = tile_rows; p.grp.num_tiles = num_tiles;
   const int n_tiles = (N + GEMM_BLOCK_N - 1) / GEMM_BLOCK_N;
-  CUtensorMap tw = ta;   // unused: records arrive by untiled bulk copies
-  const int w_by_tma = 0;
-  dim3 grid(n_tiles, max_tiles, 1);
   const uint8_t* wp = static_cast<const uint8_t*>(Wpacked);
+  // Tiles of 32 tokens and more run on pairs of SMs (32 experts of 5760 x 2880, us, before -> now: 6000 rows 389 -> 189, 1200 rows 279 -> 136, 400 rows 157 -> 130).
+  if (bt >= 32) return row_map ? -6 : LaunchPairFp4(A, lda, wp, p, bt, max_tiles, half, stream);     // (only the streaming kernel reads its rows through a map)
+  CUtensorMap ta = {};
+  if (!row_map && !MakeMapBf16(&ta, A, rows_total, K, lda, bt)) return -2;
   // 16-token tiles of the fp16 form (decode steps) go to the streaming kernel; OGB_FP4_STREAM=0 keeps them on the kernel
   // that expands through shared memory.
   static const int stream_enabled = [] { const char* e = getenv("OGB_FP4_STREAM"); return (e && e[0] == '0') ? 0 : 1; }();
-  const int skip = 0;
   if (stream_enabled && half && bt == 16 && K <= FP4_STREAM_MAX_K && max_tiles <= 65535) {
     const int stage_rows = max_rows_per_tile > 0 && max_rows_per_tile < FP4_STREAM_TOKENS ? max_rows_per_tile : FP4_STREAM_TOKENS;
     return LaunchFp4Stream(A, lda, row_map, wp, n_tiles, p, max_tiles, stage_rows, stream);
   }
-  // Tiles of 32 tokens and more run on pairs of SMs (32 experts of 5760 x 2880, us, before -> now: 6000 rows 389 -> 189, 1200 rows 279 -> 136, 400 rows 157 -> 130).
-  if (bt >= 32 && !row_map) return LaunchPairFp4(A, lda, wp, p, bt, max_tiles, half, stream);
   if (row_map) return -6;   // only the streaming kernel reads its rows through a map
-  if (bt == 16) return half ? LaunchFp4<16, true>(ta, tw, w_by_tma, wp, n_tiles, skip, p, grid, stream) : LaunchFp4<16, false>(ta, tw, w_by_tma, wp, n_tiles, skip, p, grid, stream);
-  return -5;
+  const dim3 grid(n_tiles, max_tiles, 1);
+  return half ? LaunchFp4<true>(ta, wp, n_tiles, p, grid, stream) : LaunchFp4<false>(ta, wp, n_tiles, p, grid, stream);
 }

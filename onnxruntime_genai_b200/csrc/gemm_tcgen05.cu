@@ -315,19 +315,6 @@ static bool MakeMap(CUtensorMap* out, const void* ptr, int rows, int cols, int l
   return true;
 }
 
-// A byte buffer seen as rows of 128 bytes, box = [box_rows, 128], no swizzle: one box is box_rows * 128 contiguous bytes in
-// global and in shared memory (the packed weight records of gemm_fp4.cu).
-bool MakeMapBytes128(CUtensorMap* out, const void* ptr, long long rows, int box_rows) {
-  EncodeTiledFn enc = GetEncodeTiled();
-  if (!enc || rows <= 0 || rows > 0x7fffffffll || box_rows > 256) return false;
-  cuuint64_t dims[2] = {128, cuuint64_t(rows)};
-  cuuint64_t strides[1] = {128};
-  cuuint32_t box[2] = {128, cuuint32_t(box_rows)};
-  cuuint32_t estr[2] = {1, 1};
-  return enc(out, CU_TENSOR_MAP_DATA_TYPE_UINT8, 2, const_cast<void*>(ptr), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
-             CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
-}
-
 // Shared with gemm_w4.cu (activation tensor maps).
 bool MakeMapBf16(CUtensorMap* out, const void* ptr, int rows, int cols, int ld, int box_rows) {
   return MakeMap(out, ptr, rows, cols, ld, box_rows);
