@@ -57,7 +57,7 @@ struct PairArgs {
   int bt;               // tokens of a tile: a multiple of 32 up to 256 (grouped: of the list's tiles)
   int m_tiles;          // token tiles (grouped: from the list)
   int n_pairs;          // tiles of 256 weight rows
-  int a_box;            // token rows of one copy
+  int a_box;            // token rows of one copy: half a tile
   const uint8_t* packed;
   int n_tiles;          // record tiles of 128 weight rows per k-block
 };
@@ -241,9 +241,9 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_consta
     uint32_t ph = 1;
     for (int t = first; t < total_tiles && ok; t += step) {
       const Tile x = tile_at(t);
-      const int half = cols_of(x.rows) >> 1, copies = (half + a.a_box - 1) / a.a_box;
-      const uint32_t bytes = uint32_t(copies * a.a_box * GEMM_BLOCK_K * 2 + (PACKED ? 0 : W_TILE_BYTES));
-      const int row = x.row0 + int(rank) * half, w_row = x.n_tile * GEMM_BLOCK_N;
+      // (a copy brings half of a whole tile's rows, of which a tile that ends early uses the first ones)
+      const uint32_t bytes = uint32_t(a.a_box * GEMM_BLOCK_K * 2 + (PACKED ? 0 : W_TILE_BYTES));
+      const int row = x.row0 + int(rank) * (cols_of(x.rows) >> 1), w_row = x.n_tile * GEMM_BLOCK_N;
       for (int i = 0; i < num_st; ++i) {
         const int nk = min(PAIR_KB, num_kb - i * PAIR_KB), k0 = i * (PAIR_KB * GEMM_BLOCK_K);
         if (it >= AS) ok = __all_sync(0xffffffffu, cluster_wait_bounded(&empty[s], ph, abort_flag));
@@ -265,8 +265,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_consta
           for (int h = 0; h < PAIR_KB; ++h) {
             if (h >= nk) break;
             if (!PACKED && !early) pair_tma_load_2d(stage_w(s) + h * W_TILE_BYTES, &tmap_w, bar, k0 + h * GEMM_BLOCK_K, w_row);
-            for (int c = 0; c < copies; ++c)
-              pair_tma_load_2d(stage_a(s) + h * PAIR_A_TILE + c * a.a_box * 128, &tmap_a, bar, k0 + h * GEMM_BLOCK_K, row + c * a.a_box);
+            pair_tma_load_2d(stage_a(s) + h * PAIR_A_TILE, &tmap_a, bar, k0 + h * GEMM_BLOCK_K, row);
           }
         }
         __syncwarp();

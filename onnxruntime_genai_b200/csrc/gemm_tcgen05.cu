@@ -8,7 +8,7 @@
 // swizzle written by TMA; accumulators live in tensor memory and are read back with tcgen05.ld.
 //
 // Warp roles (192 threads): warp 0 = TMA producer, warp 1 = MMA issuer, both as whole warps with one elected lane,
-// warps 2..5 = epilogue (warp 2 also owns the TMEM allocation).  A pipeline stage holds two k-blocks of 64 (see GemmCfg).
+// warps 2..5 = epilogue (warp 2 also owns the TMEM allocation).  A pipeline stage holds two k-blocks of 64, of tiles of 128 tokens and more one (see GemmCfg).
 //
 // Split-K (decode: N/128 tiles alone cannot fill 148 SMs) runs as a thread-block CLUSTER of up to
 // 8 CTAs along z: each CTA accumulates its K slice in its own tensor memory and parks the fp32 tile
@@ -569,10 +569,6 @@ OGB_API int ogb_gemm_bf16_fused(const void* A, int lda, const void* W, int ldw, 
   int kb_per = (total_kb + splits - 1) / splits;
   while (splits > 1 && kb_per * (splits - 1) >= total_kb) { --splits; kb_per = (total_kb + splits - 1) / splits; }  // no empty split
 
-  CUtensorMap tw, ta;
-  if (!MakeMap(&tw, W, N, K, ldw, GEMM_BLOCK_N)) return -2;
-  if (!MakeMap(&ta, A, M, K, lda, bt)) return -2;
-
   GemmParams p = {};
   p.M = M; p.N = N; p.K = K;
   p.splits = splits; p.kb_per_split = kb_per; p.total_kb = total_kb;
@@ -643,6 +639,9 @@ OGB_API int ogb_gemm_bf16_fused(const void* A, int lda, const void* W, int ldw, 
     if (pair_tiles > 0 || PairBf16Ns(M, N, total_kb) < waves * kb_per * (bt == 128 ? 470.0 : 420.0) + 10000.0)
       return LaunchPairBf16(A, lda, W, ldw, p, pair_tiles, stream);
   }
+  CUtensorMap tw, ta;
+  if (!MakeMap(&tw, W, N, K, ldw, GEMM_BLOCK_N)) return -2;
+  if (!MakeMap(&ta, A, M, K, lda, bt)) return -2;
   dim3 grid(n_tiles, m_tiles, splits);
   switch (bt) {
     case 16: return Launch<16>(tw, ta, p, grid, stream);
