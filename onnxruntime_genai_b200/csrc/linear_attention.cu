@@ -233,6 +233,13 @@ __global__ void __launch_bounds__(256) gdn_prepare_kernel(GdnParams<T> p, int B,
   if (h == hk * rep && lane < n) lengths[size_t(t0 + lane) * p.Hk + hk] = make_float2(pick(0, lane), pick(4, lane));
 }
 
+// A read that the compiler does not merge with an earlier one of the same place: the value is not to be kept in registers in between.
+__device__ __forceinline__ float4 ld_shared_again(uint32_t at) {
+  float4 v;
+  asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(at) : "memory");
+  return v;
+}
+
 // A thread owns two columns and NPT rows of each, 16 * NPT >= dk; the lanes of a warp are 2 column pairs x 16 row splits.  Row of split sp,
 // register i: (i / 4) * 64 + sp * 4 + i % 4, so that a thread's rows come as groups of four and the splits of a warp read two
 // 128-byte lines of a key together.  CH tokens per chunk, walked in blocks of four.
@@ -245,9 +252,14 @@ __global__ void __launch_bounds__(256) gdn_prepare_kernel(GdnParams<T> p, int B,
 // The sixteen sums of a column pair are reduced over its lanes by halving (8 + 4 + 2 + 1 shuffles, lane j ends with sum j).
 // 3001 tokens, 16 heads of 128 x 128: 1535 us with one token at a time, 1202 with all of this inside the kernel, 766 + 19 (prepare).
 // vec: rows of keys and queries start on 16 bytes and dk is a multiple of 8.
-template <typename T, int NPT, int CH>
-__global__ void __launch_bounds__(128) gated_delta_chunk_kernel(GdnParams<T> p, const float2* __restrict__ lengths, const float* __restrict__ coef, int vec) {
-  constexpr int DKP = NPT * 16, G4 = NPT / 4, LD = DKP + 4, BLK = GDN_BLOCK, NB = CH / BLK, COLS = 16;
+// WARPS: 4 columns each; CTAS: wanted per SM (0: no bound on registers); KEEP: a block's keys stay in registers for the update, else they are read again.
+// A launch that fits the GPU at once is latency bound and takes four warps with all the registers they want; one of several waves takes eight warps,
+// which stage a chunk once for 32 columns, and fewer registers (us, four / eight warps: 16 requests of 400 tokens, 32 heads of 128 x 128 1690 / 1162,
+// 8 of 40 111 / 81; one of 3001, 16 heads 810 / 1067).
+template <typename T, int NPT, int CH, int WARPS, int CTAS, bool KEEP>
+__global__ void __launch_bounds__(32 * WARPS, CTAS) gated_delta_chunk_kernel(GdnParams<T> p, const float2* __restrict__ lengths, const float* __restrict__ coef,
+                                                                             int vec) {
+  constexpr int DKP = NPT * 16, G4 = NPT / 4, LD = DKP + 4, BLK = GDN_BLOCK, NB = CH / BLK, COLS = 4 * WARPS, THREADS = 32 * WARPS;
   pdl_launch_dependents();
   pdl_wait();
   const int b = blockIdx.x, h = blockIdx.y;
@@ -273,19 +285,19 @@ __global__ void __launch_bounds__(128) gated_delta_chunk_kernel(GdnParams<T> p, 
   }
 
   // a chunk's raw keys / queries / values on their way from global memory: held in registers while the previous chunk is computed
-  constexpr int VEC = DKP / 8, U = CH * VEC / 128;         // groups of eight columns of a row; groups of keys (and of queries) per thread
-  static_assert(U * 128 == CH * VEC && NB * (GDN_COEF / 4) <= 128, "whole passes");
+  constexpr int VEC = DKP / 8, U = CH * VEC / THREADS;         // groups of eight columns of a row; groups of keys (and of queries) per thread
+  static_assert(U * THREADS == CH * VEC && NB * (GDN_COEF / 4) <= THREADS && CH % 8 == 0, "whole passes");
   const T zero = act_from<T>(0.f);
   const int first_block = t0 / BLK + b;
   struct alignas(16) Eight { T v[8]; };
   Eight raw[2 * U];
   float2 len[U];
-  T rv[CH * COLS / 128];
+  T rv[CH / 8];
   float4 rc;
   auto fetch = [&](int f0) {
 #pragma unroll
     for (int u = 0; u < U; ++u) {
-      const int idx = threadIdx.x + 128 * u, t = f0 + idx / VEC, c = (idx % VEC) * 8;
+      const int idx = threadIdx.x + THREADS * u, t = f0 + idx / VEC, c = (idx % VEC) * 8;
       const bool in = t < t1;
       len[u] = in ? lengths[size_t(t) * p.Hk + hk] : make_float2(0.f, 0.f);
       const size_t at = size_t(in ? t : t0) * p.tok_stride_qk + size_t(hk) * dk + c;
@@ -302,8 +314,8 @@ __global__ void __launch_bounds__(128) gated_delta_chunk_kernel(GdnParams<T> p, 
       }
     }
 #pragma unroll
-    for (int u = 0; u < CH * COLS / 128; ++u) {
-      const int idx = threadIdx.x + 128 * u, t = f0 + idx / COLS, c = blockIdx.z * COLS + idx % COLS;
+    for (int u = 0; u < CH / 8; ++u) {
+      const int idx = threadIdx.x + THREADS * u, t = f0 + idx / COLS, c = blockIdx.z * COLS + idx % COLS;
       rv[u] = t < t1 && c < dv ? p.v[size_t(t) * p.tok_stride_v + size_t(h) * dv + c] : zero;
     }
     const int blk = threadIdx.x / (GDN_COEF / 4);
@@ -315,7 +327,7 @@ __global__ void __launch_bounds__(128) gated_delta_chunk_kernel(GdnParams<T> p, 
     __syncthreads();                                       // the previous chunk is no longer read
 #pragma unroll
     for (int u = 0; u < U; ++u) {
-      const int idx = threadIdx.x + 128 * u, tt = idx / VEC, c = (idx % VEC) * 8;
+      const int idx = threadIdx.x + THREADS * u, tt = idx / VEC, c = (idx % VEC) * 8;
       float4* dk4 = reinterpret_cast<float4*>(&sk[tt][c]);
       float4* dq4 = reinterpret_cast<float4*>(&sq[tt][c]);
       const T* k = raw[u].v;
@@ -327,8 +339,8 @@ __global__ void __launch_bounds__(128) gated_delta_chunk_kernel(GdnParams<T> p, 
       dq4[1] = make_float4(act_f32(q[4]) * nq, act_f32(q[5]) * nq, act_f32(q[6]) * nq, act_f32(q[7]) * nq);
     }
 #pragma unroll
-    for (int u = 0; u < CH * COLS / 128; ++u) {
-      const int idx = threadIdx.x + 128 * u;
+    for (int u = 0; u < CH / 8; ++u) {
+      const int idx = threadIdx.x + THREADS * u;
       sv[idx / COLS][idx % COLS] = act_f32(rv[u]);
     }
     if (threadIdx.x < NB * (GDN_COEF / 4)) reinterpret_cast<float4*>(&scoef[0][0])[threadIdx.x] = rc;
@@ -337,7 +349,7 @@ __global__ void __launch_bounds__(128) gated_delta_chunk_kernel(GdnParams<T> p, 
     const int n = min(CH, t1 - f0);
     for (int blk = 0; blk * BLK < n; ++blk) {
       const int tt = blk * BLK;
-      float kk[BLK][NPT], val[16];
+      float kk[KEEP ? BLK : 1][KEEP ? NPT : 1], val[16];
 #pragma unroll
       for (int t = 0; t < BLK; ++t) {
         const float4* k4 = reinterpret_cast<const float4*>(sk[tt + t]) + sp;
@@ -346,7 +358,7 @@ __global__ void __launch_bounds__(128) gated_delta_chunk_kernel(GdnParams<T> p, 
 #pragma unroll
         for (int i = 0; i < G4; ++i) {
           const float4 kv = k4[i * 16], qv = q4[i * 16];
-          kk[t][4 * i] = kv.x; kk[t][4 * i + 1] = kv.y; kk[t][4 * i + 2] = kv.z; kk[t][4 * i + 3] = kv.w;
+          if constexpr (KEEP) { kk[t][4 * i] = kv.x; kk[t][4 * i + 1] = kv.y; kk[t][4 * i + 2] = kv.z; kk[t][4 * i + 3] = kv.w; }
           m0 = fmaf(c0[4 * i], kv.x, m0); m1 = fmaf(c1[4 * i], kv.x, m1); r0 = fmaf(c0[4 * i], qv.x, r0); r1 = fmaf(c1[4 * i], qv.x, r1);
           m0 = fmaf(c0[4 * i + 1], kv.y, m0); m1 = fmaf(c1[4 * i + 1], kv.y, m1); r0 = fmaf(c0[4 * i + 1], qv.y, r0); r1 = fmaf(c1[4 * i + 1], qv.y, r1);
           m0 = fmaf(c0[4 * i + 2], kv.z, m0); m1 = fmaf(c1[4 * i + 2], kv.z, m1); r0 = fmaf(c0[4 * i + 2], qv.z, r0); r1 = fmaf(c1[4 * i + 2], qv.z, r1);
@@ -395,8 +407,20 @@ __global__ void __launch_bounds__(128) gated_delta_chunk_kernel(GdnParams<T> p, 
 #pragma unroll
       for (int t = 0; t < BLK; ++t) {
         const float e0 = e[t] * d[t][0], e1 = e[t] * d[t][1];
+        if constexpr (KEEP) {
 #pragma unroll
-        for (int i = 0; i < NPT; ++i) { c0[i] = fmaf(kk[t][i], e0, c0[i]); c1[i] = fmaf(kk[t][i], e1, c1[i]); }
+          for (int i = 0; i < NPT; ++i) { c0[i] = fmaf(kk[t][i], e0, c0[i]); c1[i] = fmaf(kk[t][i], e1, c1[i]); }
+        } else {
+          const uint32_t row = smem_u32(sk[tt + t]) + sp * 16;
+#pragma unroll
+          for (int i = 0; i < G4; ++i) {
+            const float4 kv = ld_shared_again(row + i * 256);
+            c0[4 * i] = fmaf(kv.x, e0, c0[4 * i]); c1[4 * i] = fmaf(kv.x, e1, c1[4 * i]);
+            c0[4 * i + 1] = fmaf(kv.y, e0, c0[4 * i + 1]); c1[4 * i + 1] = fmaf(kv.y, e1, c1[4 * i + 1]);
+            c0[4 * i + 2] = fmaf(kv.z, e0, c0[4 * i + 2]); c1[4 * i + 2] = fmaf(kv.z, e1, c1[4 * i + 2]);
+            c0[4 * i + 3] = fmaf(kv.w, e0, c0[4 * i + 3]); c1[4 * i + 3] = fmaf(kv.w, e1, c1[4 * i + 3]);
+          }
+        }
       }
     }
   }
@@ -440,15 +464,18 @@ static bool LaunchGdnDecode(const GdnParams<T>& p, int B, int splits, cudaStream
   return p.dk % NPT == 0 ? launch_pdl(gated_delta_kernel<T, NPT, true>, grid, block, 0, s, p)
                          : launch_pdl(gated_delta_kernel<T, NPT, false>, grid, block, 0, s, p);
 }
-template <typename T, int NPT, int CH>
+template <typename T, int NPT, int CH, int WARPS, int CTAS, bool KEEP>
 static bool LaunchGdnChunk(const GdnParams<T>& p, int B, int tokens, void* scratch, cudaStream_t s) {
   float* coef = static_cast<float*>(scratch);
   float2* lengths = reinterpret_cast<float2*>(coef + gdn_blocks(tokens, B) * p.Hv * GDN_COEF);
   const int vec = p.dk % 8 == 0 && ((reinterpret_cast<uintptr_t>(p.q) | reinterpret_cast<uintptr_t>(p.k) | size_t(p.tok_stride_qk) * sizeof(T)) & 15) == 0;
   return launch_pdl(gdn_prepare_kernel<T>, dim3(unsigned(gdn_blocks(tokens, B)), (p.Hv + 7) / 8), dim3(256), 0, s, p, B, lengths, coef) &&
-         launch_pdl(gated_delta_chunk_kernel<T, NPT, CH>, dim3(B, p.Hv, (p.dv + 15) / 16), dim3(128), 0, s, p, static_cast<const float2*>(lengths),
-                    static_cast<const float*>(coef), vec);
+         launch_pdl(gated_delta_chunk_kernel<T, NPT, CH, WARPS, CTAS, KEEP>, dim3(B, p.Hv, (p.dv + 4 * WARPS - 1) / (4 * WARPS)), dim3(32 * WARPS), 0, s, p,
+                    static_cast<const float2*>(lengths), static_cast<const float*>(coef), vec);
 }
+
+// CTAs of a launch of the chunk kernel with four warps
+static long long GdnTiles(int B, int Hv, int dv) { return (long long)B * Hv * ((dv + 15) / 16); }
 
 // Bytes of scratch that a launch of the chunk kernel over `tokens` tokens of `requests` requests needs (16-byte aligned).
 OGB_API long long ogb_gated_delta_scratch_bytes(int tokens, int requests, int Hk, int Hv) {
@@ -467,9 +494,10 @@ static int LaunchGatedDelta(const GdnParams<T>& p, int B, int tokens, int max_q_
   bool ok;
   if (max_q_len != 1 && dk <= 256 && scratch) {
     if (reinterpret_cast<uintptr_t>(scratch) & 15) return -1;
-    if (dk <= 64) ok = LaunchGdnChunk<T, 4, 32>(p, B, tokens, scratch, s);
-    else if (dk <= 128) ok = LaunchGdnChunk<T, 8, 32>(p, B, tokens, scratch, s);
-    else ok = LaunchGdnChunk<T, 16, 16>(p, B, tokens, scratch, s);
+    const bool many = GdnTiles(B, p.Hv, dv) > 2 * 148;       // more than the two per SM that are resident at once
+    if (dk <= 64) ok = many ? LaunchGdnChunk<T, 4, 32, 8, 2, true>(p, B, tokens, scratch, s) : LaunchGdnChunk<T, 4, 32, 4, 1, true>(p, B, tokens, scratch, s);
+    else if (dk <= 128) ok = many ? LaunchGdnChunk<T, 8, 16, 8, 2, false>(p, B, tokens, scratch, s) : LaunchGdnChunk<T, 8, 32, 4, 0, true>(p, B, tokens, scratch, s);
+    else ok = many ? LaunchGdnChunk<T, 16, 16, 8, 1, true>(p, B, tokens, scratch, s) : LaunchGdnChunk<T, 16, 16, 4, 0, true>(p, B, tokens, scratch, s);
     return ok ? 0 : -4;
   }
   // measured at Qwen3.5 shapes: 32 rows per thread 51 us, 16 rows 63 us, 64 rows 54 us (64 requests)

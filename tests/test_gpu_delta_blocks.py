@@ -47,6 +47,29 @@ def test_blocks_follow_the_recurrence(Hk, Hv, dk, dv, lens):
     assert torch.allclose(dev_state.cpu(), state, rtol=1e-4, atol=1e-4)
 
 
+@pytest.mark.parametrize("Hk,Hv,dk,dv,B", [(2, 4, 64, 128, 11), (2, 4, 40, 65, 20), (2, 4, 128, 128, 11), (4, 4, 100, 130, 11), (2, 2, 200, 64, 40), (1, 4, 256, 128, 11)])
+@pytest.mark.parametrize("longest", [2, 5, 9, 17, 50])
+def test_many_requests(Hk, Hv, dk, dv, B, longest):
+    """More column tiles than fit the GPU at once (the form with eight warps), and portions of a few tokens, which are walked one at a time."""
+    gen = torch.Generator().manual_seed(dk + longest)
+    lens = [longest] + [int(n) for n in torch.randint(0, longest + 1, (B - 1,), generator=gen)]
+    T = sum(lens)
+    unit = lambda *s: torch.nn.functional.normalize(torch.randn(*s, generator=gen), dim=-1).to(torch.bfloat16)  # noqa: E731
+    q, k, v = unit(T, Hk, dk), unit(T, Hk, dk), torch.randn(T, Hv, dv, generator=gen).to(torch.bfloat16)
+    g, beta = -torch.rand(T, Hv, generator=gen), torch.rand(T, Hv, generator=gen)
+    state = torch.randn(B + 1, Hv, dk, dv, generator=gen) * 0.3
+    slots = torch.randperm(B + 1, generator=gen)[:B].to(torch.int32)
+    past = [3 * (r % 2) for r in range(B)]
+    cu = torch.tensor([0] + lens).cumsum(0).to(torch.int32).cuda()
+    dev_state = state.cuda()
+    got = ops.gated_delta(q.cuda(), k.cuda(), v.cuda(), g.cuda(), beta.cuda(), dev_state, slots.cuda(), cu, torch.tensor(past, dtype=torch.int32).cuda(), longest)
+    ops.check_kernel_status()
+    want = _recurrence(q, k, v, g, beta, state, lens, past, slots.tolist())
+    # as above: at most 50 tokens
+    assert ((got.cpu().double() - want).abs() <= 2.0 ** -8 * want.abs() + 1e-4).all()
+    assert torch.allclose(dev_state.cpu(), state, rtol=1e-4, atol=1e-4)
+
+
 def test_a_later_token_that_is_not_finite_leaves_earlier_ones_alone():
     gen = torch.Generator().manual_seed(5)
     T, H, d = 8, 1, 64
