@@ -296,7 +296,7 @@ int ogb_gated_delta_fused(const void* conv, long long conv_stride, long long q_o
                           float q_scale, float l2_eps, float* state, long long slot_stride, const int32_t* slots, const int32_t* cu_seqlens,
                           const int32_t* past_lens, void* out, int B, int Hk, int Hv, int dk, int dv, int tokens, int max_q_len, int fp32, void* scratch,
                           void* stream);
-long long ogb_gated_delta_scratch_bytes(int tokens, int requests, int Hk, int Hv);
+long long ogb_gated_delta_scratch_bytes(int tokens, int requests, int Hk, int Hv, int dk, int dv, int max_q_len);
 int ogb_gdn_gate_norm(const void* o, const void* z, long long z_stride, const float* w, float eps, void* out, long long out_stride, int T, int Hv,
                       int dv, int fp32, void* stream);
 int ogb_gated_delta(const void* q, const void* k, const void* v, const float* g, const float* beta, float* state, const int32_t* slots,

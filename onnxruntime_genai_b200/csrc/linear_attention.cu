@@ -4,7 +4,7 @@
 //
 // Two kernels over the same state pool (fp32, [slots][value heads][dk][dv] with a slot stride), for bf16 and fp32 activations and any
 // dk / dv (rows and columns past the sizes are zeros):
-//   gated_delta_kernel        decode-shaped steps.  One CTA = (request, value head, 32 columns of the head's state S [dk, dv]); a thread
+//   gated_delta_kernel        decode-shaped steps and portions of a few tokens.  One CTA = (request, value head, 32 columns of the head's state S [dk, dv]); a thread
 //                             keeps 16 to 64 rows of one column, the lanes of a warp are neighbouring columns (the state streams in
 //                             full lines), the row splits of a column meet in shared memory.
 //   gated_delta_chunk_kernel  prompts.  Tokens four at a time; the row splits of a column are lanes of one warp, so that dot products are
@@ -112,12 +112,13 @@ __global__ void __launch_bounds__(512) gated_delta_kernel(GdnParams<T> p) {
     }
     float decay, bt;
     gdn_gates(p, t, h, decay, bt);
-    float mem = 0.f;
+    float part[4] = {0.f, 0.f, 0.f, 0.f};                  // (four short chains: half the rounding error of one long one, and less latency)
 #pragma unroll
     for (int i = 0; i < NPT; ++i) {
       col[i] *= decay;
-      mem = fmaf(col[i], sk[n0 + i], mem);
+      part[i & 3] = fmaf(col[i], sk[n0 + i], part[i & 3]);
     }
+    float mem = (part[0] + part[1]) + (part[2] + part[3]);
     if (splits > 1) {
       sM[sp][jj] = mem;
       __syncthreads();
@@ -126,12 +127,13 @@ __global__ void __launch_bounds__(512) gated_delta_kernel(GdnParams<T> p) {
     }
     const float vj = live ? act_f32(p.v[size_t(t) * p.tok_stride_v + size_t(h) * dv + j]) : 0.f;
     const float delta = (vj - mem * rk) * bt * rk;       // the normalised key is rk * sk: once in the read, once in the write
-    float o = 0.f;
+    part[0] = part[1] = part[2] = part[3] = 0.f;
 #pragma unroll
     for (int i = 0; i < NPT; ++i) {
       col[i] = fmaf(sk[n0 + i], delta, col[i]);
-      o = fmaf(col[i], sq[n0 + i], o);
+      part[i & 3] = fmaf(col[i], sq[n0 + i], part[i & 3]);
     }
+    float o = (part[0] + part[1]) + (part[2] + part[3]);
     if (splits > 1) {
       sO[sp][jj] = o;
       __syncthreads();
@@ -476,14 +478,22 @@ static bool LaunchGdnChunk(const GdnParams<T>& p, int B, int tokens, void* scrat
 
 // CTAs of a launch of the chunk kernel with four warps
 static long long GdnTiles(int B, int Hv, int dv) { return (long long)B * Hv * ((dv + 15) / 16); }
+// Whether portions of up to max_q_len tokens (0: unknown) run in blocks.  A few tokens are walked by the decode kernel, which has no second launch and
+// stages nothing (us, blocks / walked, 32 heads of 128 x 128: one request of 2 / 5 tokens 14.3 / 8.0, 15.3 / 13.1; 32 of 2 / 8 tokens 162 / 36,
+// 182 / 100; 8 heads of 64 x 64: one of 4 / 5 10.1 / 10.2, 10.6 / 11.9; 32 of 5 / 8 23 / 14, 22 / 19; 16 heads of 128, 8 of 8 / 12 33 / 24, 38 / 33).
+// Both are 32-bit sums: 1.0e-7 to 1.3e-7 of the result's norm from 64 bits with 32-bit activations.
+static bool GdnInBlocks(int B, int Hv, int dk, int dv, int max_q_len) {
+  if (dk > 256) return false;
+  return max_q_len == 0 || max_q_len > (GdnTiles(B, Hv, dv) >= 1024 ? 8 : dk > 64 ? 5 : 4);
+}
 
-// Bytes of scratch that a launch of the chunk kernel over `tokens` tokens of `requests` requests needs (16-byte aligned).
-OGB_API long long ogb_gated_delta_scratch_bytes(int tokens, int requests, int Hk, int Hv) {
-  return (gdn_blocks(tokens, requests) * Hv * GDN_COEF + 2ll * tokens * Hk) * 4;
+// Bytes of scratch that a launch over `tokens` tokens of `requests` requests needs (16-byte aligned); 0: none.
+OGB_API long long ogb_gated_delta_scratch_bytes(int tokens, int requests, int Hk, int Hv, int dk, int dv, int max_q_len) {
+  return GdnInBlocks(requests, Hv, dk, dv, max_q_len) ? (gdn_blocks(tokens, requests) * Hv * GDN_COEF + 2ll * tokens * Hk) * 4 : 0;
 }
 
 // max_q_len: the most tokens a request of the launch feeds (1: the decode kernel; 0: unknown, treated as a prompt)
-// scratch: ogb_gated_delta_scratch_bytes(tokens, B, Hk, Hv) bytes, or null: the decode kernel walks the tokens
+// scratch: ogb_gated_delta_scratch_bytes(tokens, B, Hk, Hv, dk, dv, max_q_len) bytes, or null: the decode kernel walks the tokens
 template <typename T>
 static int LaunchGatedDelta(const GdnParams<T>& p, int B, int tokens, int max_q_len, void* scratch, void* stream) {
   if (B <= 0) return 0;
@@ -492,7 +502,7 @@ static int LaunchGatedDelta(const GdnParams<T>& p, int B, int tokens, int max_q_
   if (dk > GDN_MAX_DK) return -5;
   auto s = static_cast<cudaStream_t>(stream);
   bool ok;
-  if (max_q_len != 1 && dk <= 256 && scratch) {
+  if (scratch && GdnInBlocks(B, p.Hv, dk, dv, max_q_len)) {
     if (reinterpret_cast<uintptr_t>(scratch) & 15) return -1;
     const bool many = GdnTiles(B, p.Hv, dv) > 2 * 148;       // more than the two per SM that are resident at once
     if (dk <= 64) ok = many ? LaunchGdnChunk<T, 4, 32, 8, 2, true>(p, B, tokens, scratch, s) : LaunchGdnChunk<T, 4, 32, 4, 1, true>(p, B, tokens, scratch, s);

@@ -582,9 +582,10 @@ def causal_conv(x, weight, bias, cache, slots, positions, cu_seqlens, past_lens,
     return out
 
 
-def _gated_delta_scratch(T, B, Hk, Hv, max_q_len, device):
-    """Scratch of the recurrence's prompt kernel (lengths and block coefficients); a decode step needs none."""
-    return None if max_q_len == 1 else torch.empty(_lib.lib().ogb_gated_delta_scratch_bytes(T, B, Hk, Hv), dtype=torch.uint8, device=device)
+def _gated_delta_scratch(T, B, Hk, Hv, dk, dv, max_q_len, device):
+    """Scratch of the recurrence's prompt kernel (lengths and block coefficients); steps of a few tokens per request need none."""
+    size = _lib.lib().ogb_gated_delta_scratch_bytes(T, B, Hk, Hv, dk, dv, int(max_q_len))
+    return torch.empty(size, dtype=torch.uint8, device=device) if size else None
 
 
 def gated_delta(q, k, v, g, beta, state, slots, cu_seqlens, past_lens, max_q_len: int = 0):
@@ -600,7 +601,7 @@ def gated_delta(q, k, v, g, beta, state, slots, cu_seqlens, past_lens, max_q_len
     gf, bf = g.float().contiguous(), beta.float().contiguous()
     out = torch.empty(T, Hv, dv, dtype=torch.bfloat16, device=q.device)
     B = past_lens.shape[0]
-    scratch = _gated_delta_scratch(T, B, Hk, Hv, max_q_len, q.device)
+    scratch = _gated_delta_scratch(T, B, Hk, Hv, dk, dv, max_q_len, q.device)
     _lib.check(_lib.lib().ogb_gated_delta(_ptr(q), _ptr(k), _ptr(v), _ptr(gf), _ptr(bf), _ptr(state), _ptr(slots), _ptr(cu_seqlens), _ptr(past_lens),
                                           _ptr(out), B, Hk, Hv, dk, dv, T, int(max_q_len), _ptr(scratch), _stream()), "gated_delta")
     return out
@@ -620,7 +621,7 @@ def gated_delta_layer(conv, proj, cd, vd, Hk, Hv, dk, dv, neg_exp_a, dt_bias, no
     kd, f32 = Hk * dk, int(conv.dtype == torch.float32)
     o = torch.empty(T, Hv, dv, dtype=conv.dtype, device=conv.device)
     B = past_lens.shape[0]
-    scratch = _gated_delta_scratch(T, B, Hk, Hv, max_q_len, conv.device)
+    scratch = _gated_delta_scratch(T, B, Hk, Hv, dk, dv, max_q_len, conv.device)
     _lib.check(_lib.lib().ogb_gated_delta_fused(_ptr(conv), conv.stride(0), 0, kd, 2 * kd, _ptr(proj), proj.stride(0), cd + vd, cd + vd + Hv,
                                                 _ptr(neg_exp_a), _ptr(dt_bias), float(dk) ** -0.5, float(l2_eps), _ptr(state), state.stride(0),
                                                 _ptr(slots), _ptr(cu_seqlens), _ptr(past_lens), _ptr(o), B, Hk, Hv, dk, dv, T, int(max_q_len), f32,

@@ -12,6 +12,13 @@ def test_packed_experts_refuse_token_tiles_without_a_kernel(tile, half):
     assert _lib.lib().ogb_moe_gemm_fp4(A, 128, W, C, 256, 64, 256, 128, 4, None, half, 0, 0.0, 0.0, LIST, LIST, LIST, LIST, 8, tile, 64, None, None, None) == -5
 
 
+@pytest.mark.parametrize("requests,Hv,dk,dv,longest,blocks", [
+    (1, 16, 128, 128, 1, False), (1, 16, 128, 128, 5, False), (1, 16, 128, 128, 6, True), (1, 16, 128, 128, 0, True), (8, 16, 128, 128, 8, False),
+    (8, 16, 128, 128, 9, True), (1, 8, 64, 64, 4, False), (1, 8, 64, 64, 5, True), (32, 8, 64, 64, 8, False), (1, 4, 257, 64, 3000, False), (1, 4, 256, 64, 3000, True)])
+def test_short_portions_of_the_delta_rule_are_walked(requests, Hv, dk, dv, longest, blocks):
+    assert (_lib.lib().ogb_gated_delta_scratch_bytes(requests * max(1, longest), requests, Hv // 2, Hv, dk, dv, longest) > 0) == blocks
+
+
 @pytest.mark.parametrize("M,N,K,splits", [(129, 512, 14336, 8), (512, 512, 14336, 8), (300, 128, 8192, 8), (200, 896, 4864, 8), (257, 896, 4864, 8), (200, 2048, 8192, 4),
                                           (257, 1024, 14336, 4), (64, 4096, 4096, 4)])
 def test_long_sums_of_few_tiles_are_cut_in_eight(M, N, K, splits):
