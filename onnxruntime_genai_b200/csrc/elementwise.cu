@@ -606,7 +606,7 @@ OGB_API int ogb_rope_kv_append_bits(void* qkv, int qkv_stride, const int32_t* po
   // The vector form addresses groups of 8 columns: head sizes and rotated parts of whole pairs of groups, rows and caches that start on 16 bytes.
   const uintptr_t base = reinterpret_cast<uintptr_t>(qkv) | reinterpret_cast<uintptr_t>(k_cache) | reinterpret_cast<uintptr_t>(v_cache) |
                          reinterpret_cast<uintptr_t>(cos_cache) | reinterpret_cast<uintptr_t>(sin_cache);
-  if (!q_norm_w && !k_norm_w && !interleaved && !p.kv8 && !positions3 && D % 16 == 0 && rot % 16 == 0 && qkv_stride % 8 == 0 && base % 16 == 0) {
+  if (!q_norm_w && !k_norm_w && !interleaved && !p.kv8 && !positions3 && D >= 16 && D % 16 == 0 && rot % 16 == 0 && qkv_stride % 8 == 0 && base % 16 == 0) {
     const int per_cta = 4 * (ROPE_VEC_THREADS / (D / 16));       // heads of one pass; few tokens: a CTA per pass
     const int passes = (Hq + 2 * Hkv + per_cta - 1) / per_cta;
     return launch_pdl(rope_kv_vec_kernel, dim3(unsigned(T), unsigned(T < 64 ? passes : 1)), dim3(ROPE_VEC_THREADS), 0, static_cast<cudaStream_t>(stream), p) ? 0 : -4;

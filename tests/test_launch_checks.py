@@ -24,3 +24,8 @@ def test_short_portions_of_the_delta_rule_are_walked(requests, Hv, dk, dv, longe
 def test_long_sums_of_few_tiles_are_cut_in_eight(M, N, K, splits):
     """Of 256-token tiles, as many clusters of eight CTAs as are resident at once."""
     assert _lib.lib().ogb_gemm_auto_splits(M, N, K, 0, 148) == splits
+
+
+def test_rotation_of_heads_without_columns_does_nothing():
+    """A head size of 0 has nothing to rotate or to append: the call returns (where there is no device, with the launch's error)."""
+    assert _lib.lib().ogb_rope_kv_append_bits(A, 8, None, None, None, None, None, None, None, None, 1e-6, 1, 2, 1, 0, 0, 0, 1, 16, None, 0, 0, None) in (0, -4)
