@@ -379,7 +379,9 @@ def linear(x, w, bias=None, residual=None, out_fp32=False, out=None, splits=0, a
     reduce_scatter=(rank, world): the sum is scattered by token rows instead (sequence-parallel form): the result has
     this rank's rows [rank * ceil(T / world), ...) only, and `residual` is that slice.
     norm_eps > 0: an RMS norm folded into the GEMM - x holds the un-normalised rows, w already carries the norm's weight
-    (w * norm_weight along K), and row m of the product is scaled by rsqrt(mean(x[m]^2) + norm_eps)."""
+    (w * norm_weight along K), and row m of the product is scaled by rsqrt(mean(x[m]^2) + norm_eps).
+    splits: 0 leaves the kernel to the launcher; n > 0 asks for the one that cuts k in n parts, n < 0 for the one on pairs of SMs with -n token
+    tiles where it can take the product (no reduction over ranks, no folded norm)."""
     if isinstance(w, W4Weight):
         if norm_eps > 0:
             x = rms_scale(x, norm_eps)
@@ -490,7 +492,7 @@ _PAIR_FLAGS = {"silu": 0, "relu": GEMM_PAIR_RELU, "gelu_tanh": GEMM_PAIR_GELU, "
 
 def gate_up_act(x, w, bias=None, act="silu", out=None, splits=0, interleaved=False, norm_eps=0.0):
     """act(x @ Wg.T) * (x @ Wu.T).  w is [2I, K]: stacked [Wg; Wu], or (interleaved=True) blocks of 64 gate
-    rows + 64 up rows as produced by interleave_gate_up (the layout the fused kernel needs).  norm_eps: as in `linear`."""
+    rows + 64 up rows as produced by interleave_gate_up (the layout the fused kernel needs).  norm_eps, splits: as in `linear`."""
     fused = None
     if norm_eps > 0:
         if not x.is_cuda:
